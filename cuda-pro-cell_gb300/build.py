@@ -52,14 +52,14 @@ def build(verbose: bool = False, out: str | None = None, defines=()) -> str:
     os.makedirs(OUT, exist_ok=True)
     cuda = _cuda_home()
     nvcc = os.path.join(cuda, "bin", "nvcc")
-    headers = [os.path.join(CSRC, h) for h in ("pc_rng.h", "pc_engine.h", "pc_sweeps.cuh", "pc_guard.h")] + \
+    headers = [os.path.join(CSRC, h) for h in ("pc_rng.h", "pc_engine.h", "pc_sweeps.cuh", "pc_walk.cuh", "pc_guard.h")] + \
         [os.path.join(INCLUDE, "procell.h")]
     host_flags = ["-O2", "-std=c++17", "-fPIC", "-pthread", "-ffp-contract=off", "-fno-fast-math", "-Wall",
                   "-I" + os.path.join(cuda, "include"), "-I" + INCLUDE]
     jobs = []
     objs = []
     dflags = ["-D" + d for d in defines]
-    for name in ("pc_kernels.cu", "pc_tuned_plain.cu", "pc_tuned_batched.cu", "pc_noalloc.cu", "pc_smooth.cu"):
+    for name in ("pc_kernels.cu", "pc_tuned_plain.cu", "pc_tuned_batched.cu", "pc_walk.cu", "pc_noalloc.cu", "pc_smooth.cu"):
         k_src = os.path.join(CSRC, name)
         k_obj = os.path.join(OUT, name.replace(".cu", ".o"))
         objs.append(k_obj)

@@ -64,6 +64,12 @@ struct pc_context {
   // resident blocks per SM of each configuration's kernels: [narrow][batched][config]
   int occ[2][2][kNumSweepConfigs][3] = {};
   uint32_t* persist_ctl = nullptr;       // [2] barrier + [8] run totals (u64 [4])
+  // tree walk: control words, the warps' global regions (grown on demand; runs of one context
+  // follow one another), resident blocks per SM of its kernels [batched]
+  WalkCtl* walk_ctl = nullptr;
+  void* walk_dev = nullptr;
+  size_t walk_bytes = 0;
+  int walk_occ[2] = {0, 0};
   // the two large per-plan device buffers (root records, count table) of destroyed plans,
   // kept for the next plans of this context: two of each kind, the largest (the consecutive
   // sub-batches of pc_simulate_batch alternate between two live plans)
@@ -112,6 +118,7 @@ struct InstanceHost {
   std::vector<uint32_t> sorted_to_file;
   uint32_t fallback = 0, gmax = 0;
   double t_max = 0.0, phi = 0.0;
+  bool walkable = false;          // every type in the range of the tree walk's error bound
   uint64_t seed = 0, roots = 0;
   // placement in the plan
   uint64_t root_begin = 0, class_begin = 0;
@@ -144,8 +151,11 @@ struct pc_plan {
   pc_context* owner = nullptr;                // receives the large buffers on destroy
   size_t rec_bytes = 0, hist_bytes = 0;
   cudaGraphExec_t graph = nullptr;           // persistent driver: the captured run
-  PersistArgs graph_args;                    // ... and the arguments it was captured with
-  int graph_config = -1, graph_grid = 0;
+  // ... and what it was captured with: the launch's arguments (the persistent sweeps' or the
+  // tree walk's), configuration (-1: the tree walk) and grid
+  PersistArgs graph_args;
+  WalkArgs graph_walk;
+  int graph_config = -2, graph_grid = 0;
   pc_stats stats;
   uint64_t upload_bytes = 0;
   bool ran = false;
@@ -440,6 +450,35 @@ KeyLayout key_layout(uint64_t roots, uint32_t gmax, bool batched, uint64_t max_r
 void host_truncation_bounds(double mu, double sigma, float& zlo, float& zhi) {
   truncation_bounds(mu, sigma, zlo, zhi);
 }
+
+// The error bound of the tree walk's FP32 time left. With u = 2^-24 and every quantity a normal
+// float (or 0):
+//   timer        tau~ = fl(sd~ z + mean~): |tau~ - tau| <= u (|sd z| + mean + |tau|), and
+//                |sd z| <= mean + tau for tau > 0, so at most 2 u (mean + tau);
+//   initial cell p~ = fl(tau~ fl(1 + U~)), U~ the first 24 bits of U: 1 + U~ off by 2 u, p~ by
+//                4 u (mean + tau) + 2 u tau + u p, rem~ = fl(t~ - p~) by u t_max + u |rem| more;
+//   a daughter   rem~ = fl(rem~ - tau~): 2 u (mean + tau) + u |rem| more.
+// A lineage still in time has tau <= p <= t_max, its timers add up to at most t_max and every
+// |rem| <= t_max, so after at most `cap` divisions the error is below
+//   u (4 mean + 8 t_max) + 2 u t_max + cap u (2 mean + t_max);
+// the daughter being decided adds 2 u (mean + tau) + u |rem| with tau <= t_max + |rem|, i.e.
+// 2 u (mean + t_max) + 3 u |rem|. The rounding of the FP64 due times (2^-53) and the factor
+// 1 / (1 - 3 u) are inside the 1% on top.
+// An FP32 timer is positive in FP64 as well when it exceeds its own error at tau near 0.
+bool host_walk_type(TypeDev& t, double mean, double sd, double t_max) {
+  const double lo = 0x1p-60, hi = 0x1p60, u = 0x1p-24 * 1.01;
+  t.w_cum = t.cum <= 0.0 ? 0 : (t.cum >= 1.0 ? 1ull << 53 : (uint64_t)std::ceil(std::ldexp(t.cum, 53)));
+  if (!(t_max == 0.0 || t_max >= lo) || !(t_max <= hi)) return false;
+  if (t.mode == kModeQuiescent) return true;
+  const bool zero = t.mode == kModeZeroMean;
+  if (!zero && !(mean >= lo && mean <= hi && std::fabs(sd) <= hi)) return false;
+  t.w_mean = zero ? 0.0f : (float)mean;
+  t.w_sd = zero ? 0.0f : (float)sd;
+  t.w_eps = zero ? -1.0f : (float)(4.0 * u * mean);  // a zero-mean type's timer is 0 and not truncated
+  t.w_band_gen = (float)(u * (2.0 * mean + t_max));
+  t.w_band = (float)(u * (6.0 * mean + 13.0 * t_max));
+  return true;
+}
 }  // namespace pc
 
 extern "C" {
@@ -478,6 +517,7 @@ int pc_create(pc_context** out, int device) {
   if ((e = pc_cuda_malloc(&ctx->stats_dev, 4 * sizeof(unsigned long long))) != cudaSuccess) return bail(e, "cudaMalloc");
   if ((e = pc_cuda_malloc(&ctx->error_dev, sizeof(uint32_t))) != cudaSuccess) return bail(e, "cudaMalloc");
   if ((e = pc_cuda_malloc(&ctx->persist_ctl, 48)) != cudaSuccess) return bail(e, "cudaMalloc");
+  if ((e = pc_cuda_malloc(&ctx->walk_ctl, sizeof(WalkCtl))) != cudaSuccess) return bail(e, "cudaMalloc");
   if ((e = pc_cuda_malloc_host(&ctx->pinned, 64 * sizeof(unsigned long long))) != cudaSuccess)
     return bail(e, "cudaMallocHost");
   for (auto& ev : ctx->ev)
@@ -508,6 +548,8 @@ void pc_destroy(pc_context* ctx) {
   pc_cuda_free(ctx->stats_dev);
   pc_cuda_free(ctx->error_dev);
   pc_cuda_free(ctx->persist_ctl);
+  pc_cuda_free(ctx->walk_ctl);
+  pc_cuda_free(ctx->walk_dev);
   cudaFreeHost(ctx->pinned);
   cudaFreeHost(ctx->stage);
   cudaFreeHost(ctx->stage2);
@@ -602,6 +644,7 @@ int prepare_types(const pc_cell_type* types, uint32_t n_types, InstanceHost& I, 
   std::stable_sort(order.begin(), order.end(),
                    [&](uint32_t a, uint32_t b) { return types[a].ratio > types[b].ratio; });
   double acc = 0.0;
+  I.walkable = true;
   for (uint32_t s = 0; s < n_types; ++s) {
     const pc_cell_type& src = types[order[s]];
     TypeDev t;
@@ -620,6 +663,7 @@ int prepare_types(const pc_cell_type* types, uint32_t n_types, InstanceHost& I, 
       t.zlo = -INFINITY;
       t.zhi = INFINITY;
     }
+    if (!host_walk_type(t, src.mean, src.sd, I.t_max)) I.walkable = false;
     I.types.push_back(t);
     I.sorted_to_file.push_back(order[s]);
   }
@@ -889,7 +933,6 @@ int finalize_device(pc_context* ctx, pc_plan* p, const PlanTables& t) {
   const auto& bin_class = t.bin_class;
   const auto& btypes = t.btypes;
   const auto& idev = t.idev;
-  const uint64_t chunk = p->chunk;
   PC_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
   const size_t nb = p->nbins;
@@ -925,9 +968,6 @@ int finalize_device(pc_context* ctx, pc_plan* p, const PlanTables& t) {
       p->bin_class_dev = reinterpret_cast<uint32_t*>(base + o_bclass);
     }
   }
-  if (e == cudaSuccess)
-    e = take_spare(ctx->spare_rec, std::max<uint64_t>(1, chunk) * sizeof(unsigned long long),
-                   reinterpret_cast<void**>(&p->root_rec_dev), &p->rec_bytes);
   if (e == cudaSuccess)
     e = take_spare(ctx->spare_hist, p->hist_elems * sizeof(unsigned long long),
                    reinterpret_cast<void**>(&p->hist_dev), &p->hist_bytes);
@@ -1482,6 +1522,29 @@ int enqueue_persistent(pc_context* ctx, pc_plan* p, const SweepKernels& K, const
   return PC_OK;
 }
 
+// Captures `enqueue(stream)` into the plan's graph; *captured = false where a capture or its
+// instantiation is not possible (the caller then enqueues the same operations directly).
+template <class F>
+int capture_graph(pc_context* ctx, pc_plan* p, F&& enqueue, bool* captured) {
+  if (p->graph) cudaGraphExecDestroy(p->graph);
+  p->graph = nullptr;
+  cudaStream_t cap_st = ctx->own_stream;
+  PC_CUDA(ctx, pc_cuda_sync(ctx->stream));
+  PC_CUDA(ctx, cudaStreamBeginCapture(cap_st, cudaStreamCaptureModeThreadLocal));
+  const int rc = enqueue(cap_st);
+  cudaGraph_t g = nullptr;
+  const cudaError_t ee = cudaStreamEndCapture(cap_st, &g);
+  cudaError_t ei = cudaErrorUnknown;
+  if (rc == PC_OK && ee == cudaSuccess) ei = cudaGraphInstantiate(&p->graph, g, 0);
+  if (g) cudaGraphDestroy(g);
+  *captured = rc == PC_OK && ee == cudaSuccess && ei == cudaSuccess;
+  if (!*captured) {
+    (void)cudaGetLastError();
+    p->graph = nullptr;
+  }
+  return PC_OK;
+}
+
 // The persistent driver: the whole run as one cooperative launch (optionally replayed from
 // a captured CUDA graph). Returns PC_ERR_UNSUPPORTED when the plan needs more level
 // buffers than the kernel's schedule holds (the caller then uses the host driver).
@@ -1539,27 +1602,12 @@ int run_persistent(pc_context* ctx, pc_plan* p, const SweepKernels& K, const int
     const bool same = p->graph && p->graph_config == ctx->opt_config && p->graph_grid == grid &&
                       std::memcmp(&p->graph_args, &pa, sizeof(pa)) == 0;
     if (!same) {
-      if (p->graph) cudaGraphExecDestroy(p->graph);
-      p->graph = nullptr;
-      cudaStream_t cap_st = ctx->own_stream;
-      PC_CUDA(ctx, pc_cuda_sync(st));
-      PC_CUDA(ctx, cudaStreamBeginCapture(cap_st, cudaStreamCaptureModeThreadLocal));
-      rc = enqueue_persistent(ctx, p, K, pa, grid, cap_st);
-      cudaGraph_t g = nullptr;
-      const cudaError_t ee = cudaStreamEndCapture(cap_st, &g);
-      cudaError_t ei = cudaErrorUnknown;
-      if (rc == PC_OK && ee == cudaSuccess) ei = cudaGraphInstantiate(&p->graph, g, 0);
-      if (g) cudaGraphDestroy(g);
-      if (rc != PC_OK || ee != cudaSuccess || ei != cudaSuccess) {
-        // capture or instantiation not possible here: run the same operations directly
-        (void)cudaGetLastError();
-        p->graph = nullptr;
-        use_graph = false;
-      } else {
-        p->graph_args = pa;
-        p->graph_config = ctx->opt_config;
-        p->graph_grid = grid;
-      }
+      rc = capture_graph(ctx, p, [&](cudaStream_t s) { return enqueue_persistent(ctx, p, K, pa, grid, s); },
+                         &use_graph);
+      if (rc != PC_OK) return rc;
+      p->graph_args = pa;
+      p->graph_config = ctx->opt_config;
+      p->graph_grid = grid;
     }
   }
   if (use_graph) {
@@ -1579,6 +1627,125 @@ int run_persistent(pc_context* ctx, pc_plan* p, const SweepKernels& K, const int
   p->stats.device_ms = ms;
   p->stats.divide_ms = ms;  // root and division sweeps share the launch
   p->stats.d2h_bytes = 72u;
+  return PC_OK;
+}
+
+// Whether a run goes to the tree walk: phi caps up to kWalkMaxGen, every type in the range of its
+// error bound, the default sweep configuration, and no cap on the size of a sweep (those
+// options, and the other configurations, ask for level sweeps).
+bool walk_serves(const pc_context* ctx, const pc_plan* p) {
+  if (p->gmax > kWalkMaxGen || ctx->opt_config != kDefaultSweepConfig) return false;
+  if (ctx->opt_max_slice || ctx->opt_max_root_chunk) return false;
+  for (const InstanceHost& I : p->inst)
+    if (!I.walkable) return false;
+  return true;
+}
+
+// The operations of one tree walk, in stream order (also what a graph captures).
+int enqueue_walk(pc_context* ctx, pc_plan* p, const WalkArgs& w, int grid, cudaStream_t s) {
+  PC_CUDA(ctx, pc_cuda_memset(p->hist_dev, 0, p->hist_elems * sizeof(unsigned long long), s));
+  PC_CUDA(ctx, pc_cuda_memset(ctx->walk_ctl, 0, sizeof(WalkCtl), s));
+  PC_CUDA(ctx, PC_LAUNCH(launch_walk(w, grid, s)));
+  PC_CUDA(ctx, pc_cuda_copy(ctx->pinned + 24, ctx->walk_ctl, offsetof(WalkCtl, barrier), cudaMemcpyDeviceToHost, s));
+  return PC_OK;
+}
+
+// The whole run as one tree walk (with the persistent driver optionally replayed from a
+// captured CUDA graph). PC_ERR_UNSUPPORTED when it does not serve this run.
+int run_walk(pc_context* ctx, pc_plan* p, const RunArgs& a) {
+  cudaStream_t st = ctx->stream;
+  int& occ = ctx->walk_occ[p->batched ? 1 : 0];
+  if (occ == 0) {
+    int n = 0;
+    const int e = walk_occupancy(p->batched, &n);
+    if (e != 0) return fail(ctx, PC_ERR_CUDA, std::string("occupancy query: ") + cudaGetErrorString((cudaError_t)e));
+    occ = std::max(1, n);
+  }
+  const int grid = max_blocks(ctx, occ);
+  const uint64_t nroots = p->root_end - p->root_begin;
+  const uint64_t warps = (uint64_t)grid * walk_warps_per_block();
+  if (nroots >= 0xFFFFFFFFull - warps) return PC_ERR_UNSUPPORTED;  // supplies are numbered in 32 bits
+  WalkArgs w;
+  std::memset(&w, 0, sizeof(w));
+  w.a = a;
+  w.a.root_rec = nullptr;
+  w.a.rec_cap = 0;
+  w.a.stats = nullptr;
+  w.a.error = &ctx->walk_ctl->error;
+  w.ctl = ctx->walk_ctl;
+  w.root_lo = p->root_begin;
+  w.root_hi = p->root_end;
+  w.batch = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(4, (nroots + warps - 1) / warps));
+  // initial cells of a range share bins, hence window columns; small enough that the ranges
+  // still deal the work out evenly
+  w.chunk = (uint32_t)std::min<uint64_t>(256, std::max<uint64_t>(w.batch, nroots / (warps * 4) / 32 * 32));
+  w.timeout_ns = 60000000000ull;
+  // a stack holds at most about 32 cells per generation; a region that overflows all the same
+  // sets an error bit and the run goes to the level sweeps
+  w.region_stride = 32ull * (p->gmax + 2u) + 512u;
+  const size_t per_warp = 2 * (w.region_stride * sizeof(uint4) + 2 * kWalkCols * sizeof(uint4) + sizeof(uint4) +
+                               sizeof(ulonglong2));
+  const size_t need = warps * per_warp;
+  if ((double)need > budget_bytes(ctx)) return PC_ERR_UNSUPPORTED;
+  if (ctx->walk_bytes < need) {
+    PC_CUDA(ctx, pc_cuda_sync(st));
+    pc_cuda_free(ctx->walk_dev);
+    ctx->walk_dev = nullptr;
+    ctx->walk_bytes = 0;
+    PC_CUDA(ctx, pc_cuda_malloc(&ctx->walk_dev, need));
+    ctx->walk_bytes = need;
+  }
+  char* at = static_cast<char*>(ctx->walk_dev);
+  auto place = [&at](size_t bytes) {
+    char* r = at;
+    at += bytes;
+    return r;
+  };
+  for (int i = 0; i < 2; ++i) {
+    w.region[i] = reinterpret_cast<uint4*>(place(warps * w.region_stride * sizeof(uint4)));
+    w.cols[i] = reinterpret_cast<uint4*>(place(warps * 2 * kWalkCols * sizeof(uint4)));
+    w.sources[i] = reinterpret_cast<uint4*>(place(warps * sizeof(uint4)));
+    w.ranges[i] = reinterpret_cast<ulonglong2*>(place(warps * sizeof(ulonglong2)));
+  }
+
+  float ms = 0.f;
+  PC_CUDA(ctx, pc_cuda_event_record(ctx->ev[0], st));
+  bool use_graph = ctx->opt_driver == 1 && ctx->opt_graph != 0;
+  int rc = PC_OK;
+  if (use_graph) {
+    const bool same = p->graph && p->graph_config == -1 && p->graph_grid == grid &&
+                      std::memcmp(&p->graph_walk, &w, sizeof(w)) == 0;
+    if (!same) {
+      rc = capture_graph(ctx, p, [&](cudaStream_t s) { return enqueue_walk(ctx, p, w, grid, s); }, &use_graph);
+      if (rc != PC_OK) return rc;
+      p->graph_walk = w;
+      p->graph_config = -1;
+      p->graph_grid = grid;
+    }
+  }
+  if (use_graph) {
+    PC_CUDA(ctx, pc_cuda_graph_launch(p->graph, st));
+  } else {
+    rc = enqueue_walk(ctx, p, w, grid, st);
+    if (rc != PC_OK) return rc;
+  }
+  PC_CUDA(ctx, pc_cuda_event_record(ctx->ev[1], st));
+  PC_CUDA(ctx, pc_cuda_sync(st));
+  PC_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]));
+  WalkCtl c;
+  std::memcpy(&c, ctx->pinned + 24, offsetof(WalkCtl, barrier));
+  if (c.error & kErrWalkStack) return PC_ERR_UNSUPPORTED;
+  p->stats.divisions = c.divisions;
+  p->stats.sweeps = c.rounds;
+  p->stats.max_generation = c.max_gen;
+  p->stats.root_sweeps = 1;
+  p->stats.kernel_launches = 1;
+  p->stats.device_ms = ms;
+  p->stats.divide_ms = ms;  // initial cells and divisions share the launch
+  p->stats.d2h_bytes = offsetof(WalkCtl, barrier);
+  ctx->pinned[0] = c.vanished;
+  ctx->pinned[1] = c.uncounted;
+  ctx->pinned[8] = c.error;
   return PC_OK;
 }
 
@@ -1649,19 +1816,30 @@ int pc_plan_run(pc_context* ctx, pc_plan* p) {
   p->ran = true;
   ++p->run_id;
   const bool narrow = p->gmax <= kNarrowMaxGen;
+  const bool empty = nroots == 0 || p->nbins == 0;
+  RunArgs a = make_args(ctx, p);
+  int rc = PC_ERR_UNSUPPORTED;
+  if (!empty && walk_serves(ctx, p)) rc = run_walk(ctx, p, a);
   const int config = narrow ? ctx->opt_config : kDefaultSweepConfig;
   const SweepKernels& K = sweep_kernels(narrow, p->batched, config);
   int occ[3];
-  int rc = kernel_occupancy(ctx, narrow, p->batched, config, K, occ);
-  if (rc != PC_OK) return rc;
-  RunArgs a = make_args(ctx, p);
-  rc = PC_ERR_UNSUPPORTED;
-  if (ctx->opt_driver == 1 && nroots > 0 && p->nbins > 0) rc = run_persistent(ctx, p, K, occ, a);
+  if (rc == PC_ERR_UNSUPPORTED) {
+    // the level sweeps, which keep a record per initial cell of a chunk
+    const int ro = kernel_occupancy(ctx, narrow, p->batched, config, K, occ);
+    if (ro != PC_OK) return ro;
+    if (!p->root_rec_dev) {
+      PC_CUDA(ctx, take_spare(ctx->spare_rec, std::max<uint64_t>(1, p->chunk) * sizeof(unsigned long long),
+                              reinterpret_cast<void**>(&p->root_rec_dev), &p->rec_bytes));
+      a.root_rec = p->root_rec_dev;
+      a.rec_cap = p->rec_bytes / sizeof(unsigned long long);
+    }
+    if (ctx->opt_driver == 1 && !empty) rc = run_persistent(ctx, p, K, occ, a);
+  }
   if (rc == PC_ERR_UNSUPPORTED) {
     PC_CUDA(ctx, pc_cuda_memset(p->hist_dev, 0, p->hist_elems * sizeof(unsigned long long), st));
     PC_CUDA(ctx, pc_cuda_memset(ctx->stats_dev, 0, 4 * sizeof(unsigned long long), st));
     PC_CUDA(ctx, pc_cuda_memset(ctx->error_dev, 0, sizeof(uint32_t), st));
-    if (nroots == 0 || p->nbins == 0) {
+    if (empty) {
       PC_CUDA(ctx, pc_cuda_sync(st));
       return PC_OK;
     }
@@ -1906,6 +2084,7 @@ int pc_batch_set_types(pc_context* ctx, pc_batch* b, const pc_cell_type* types) 
     I.types.swap(next[i].types);
     I.sorted_to_file.swap(next[i].sorted_to_file);
     I.fallback = next[i].fallback;
+    I.walkable = next[i].walkable;
   }
   std::vector<BatchType> btypes;
   std::vector<InstanceDev> idev;
@@ -2152,7 +2331,7 @@ int pc_autotune(pc_context* ctx, pc_plan* p, uint32_t repeats, pc_tuning* out) {
     }
   // within 1% (the spread of single timings) the persistent driver wins: one graph-replayed
   // launch per run and no host round trip per sweep
-  if (best_drv == 0 && best_persist <= 1.01 * best) {
+  if (best_drv == 0 && best_persist <= 1.01 * best && best_persist <= dflt) {
     best = best_persist;
     best_cfg = persist_cfg;
     best_drv = 1;

@@ -67,20 +67,27 @@ struct alignas(16) TypeDev {
   double cum;        // 32: cumulative ratio in this order
   int32_t mode;      // 40
   int32_t pad;
+  // the tree walk's form of the type (pc_walk.cuh; host_walk_type fills it)
+  float w_mean, w_sd;   // 48: mean, sd
+  float w_eps;          // 56: an FP32 timer above it is certainly positive in FP64
+  float w_band_gen;     // 60: error of the time left per generation of the phi cap
+  float w_band;         // 64: ... and of the initial cell and the last step
+  uint32_t w_pad;
+  uint64_t w_cum;       // 72: u < cum on the uniform's 53-bit integer
 };
 
 // Batched form: the parameters of one type together with its instance's (one table
 // entry per type of every instance, in instance order).
-// The division sweep reads bytes 0-31 (type, t_max) and 48-63 (seed, first cell) as three
+// The division sweep reads bytes 0-31 (type, t_max) and 80-95 (seed, first cell) as three
 // 16-byte loads.
 struct alignas(16) BatchType {
-  TypeDev t;            // bytes 0-47
-  uint32_t k0, k1;      // 48: the instance's seed
-  uint64_t root_begin;  // 56: the instance's first initial cell in the batch
-  uint32_t instance;    // 64
+  TypeDev t;            // bytes 0-79
+  uint32_t k0, k1;      // 80: the instance's seed
+  uint64_t root_begin;  // 88: the instance's first initial cell in the batch
+  uint32_t instance;    // 96
   uint32_t pad[3];
 };
-static_assert(sizeof(TypeDev) == 48 && sizeof(BatchType) == 80, "layout read by the division sweep");
+static_assert(sizeof(TypeDev) == 80 && sizeof(BatchType) == 112, "layout read by the division sweep");
 
 struct InstanceDev {
   uint32_t type_begin, ntypes, fallback, pad;
@@ -107,7 +114,8 @@ struct RunArgs {
   unsigned long long* stats; // [0] vanished, [1] uncounted, [2] max generation
   uint32_t* error;           // bit 0: depth overflow, bit 1: sampler round budget exhausted,
                              // bit 2: grid barrier timeout, bit 3: persistent schedule out of
-                             // buffers, bit 4: a bounds check of the checked build failed
+                             // buffers, bit 4: a bounds check of the checked build failed,
+                             // bit 5: a tree walk's stack outgrew its region
   uint32_t nclass;           // histogram classes per generation
   // batched form only (null otherwise)
   const BatchType* btypes;   // [all types]
@@ -153,6 +161,45 @@ struct PersistArgs {
   unsigned long long* out;          // [4] divisions, sweeps, max generation, chunks
   unsigned long long timeout_ns;    // a grid barrier waiting longer sets error bit 2
 };
+
+// The tree walk (pc_walk.cuh): a whole run in one cooperative launch. Serves phi caps up to
+// kWalkMaxGen and types and t_max in the range of its error bound (host_walk_type).
+constexpr uint32_t kWalkCols = 16;       // histogram classes in a warp's shared-memory window
+constexpr uint32_t kWalkMaxGen = 31;     // deepest phi cap it serves (32-bit nodes, window words per class)
+constexpr uint32_t kErrWalkStack = 32u;  // error bit 5
+
+// Control words of one round (zero before it).
+struct WalkRound {
+  unsigned long long handed;  // warps that handed cells over << 32 | cells handed over
+  uint32_t next;              // supplies taken beyond every warp's first
+  uint32_t idle;              // warps that have finished the round
+  uint32_t ranges, pad;       // ranges of initial cells given back
+};
+struct WalkCtl {
+  unsigned long long divisions, vanished, uncounted;
+  uint32_t max_gen, rounds;
+  uint32_t error, pad;
+  uint32_t barrier[2];
+  WalkRound round[4];  // round r uses r mod 4
+};
+
+struct WalkArgs {
+  RunArgs a;                     // root_rec, stats and the level geometry unused
+  WalkCtl* ctl;
+  uint64_t root_lo, root_hi;     // initial cells of the run
+  uint32_t chunk;                // initial cells a warp takes at once
+  uint32_t batch;                // ... and walks at once, at most 32
+  uint4* region[2];              // [warps][region_stride] cells spilled or handed over, by round parity
+  uint64_t region_stride;
+  uint4* cols[2];                // [warps][2 kWalkCols] the column tables of the cells handed over
+  uint4* sources[2];             // [warps] {warp, cells, columns, first cell}
+  ulonglong2* ranges[2];         // [warps] ranges of initial cells given back
+  unsigned long long timeout_ns; // grid barrier limit
+};
+
+int walk_occupancy(bool batched, int* blocks_per_sm);
+uint32_t walk_warps_per_block();
+int launch_walk(const WalkArgs& w, int blocks, void* stream);  // cooperative launch
 
 // One compiled configuration of the sweeps (the autotuner's search space): threads per
 // block, input cells per lane per step, and where leaf counts are privatised (a window of
@@ -262,6 +309,9 @@ int launch_smooth_gauss_newton(const SmoothArgs& A, const double* params, uint32
 // Host helpers (pc_api.cpp).
 ZigTables host_zig_tables();
 void host_truncation_bounds(double mu, double sigma, float& zlo, float& zhi);
+// Fills the tree walk's fields of a type whose mean, sd (unscaled), cum and mode are given;
+// false when the type or t_max is outside the range of the walk's error bound.
+bool host_walk_type(TypeDev& t, double mean, double sd, double t_max);
 
 // The output value set a plan builds for this histogram and phi (0: automatic), ascending,
 // into values[capacity]; PC_ERR_INVALID (with *n_values set) when it does not fit.

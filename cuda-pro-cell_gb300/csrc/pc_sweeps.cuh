@@ -180,15 +180,15 @@ __device__ __forceinline__ TypeCtx type_ctx(const RunArgs& a, const TypeDev* sme
   TypeCtx c;
   if (Batched) {
     const uint4* q = reinterpret_cast<const uint4*>(a.btypes + ty);
-    const uint4 q0 = __ldg(q), q1 = __ldg(q + 1), q3 = __ldg(q + 3);
+    const uint4 q0 = __ldg(q), q1 = __ldg(q + 1), q5 = __ldg(q + 5);
     c.mu = __hiloint2double((int)q0.y, (int)q0.x);
     c.sigma = __hiloint2double((int)q0.w, (int)q0.z);
     c.zlo = __uint_as_float(q1.x);
     c.zhi = __uint_as_float(q1.y);
     c.t_max = __hiloint2double((int)q1.w, (int)q1.z);
-    c.k0 = q3.x;
-    c.k1 = q3.y;
-    c.root_begin = ((uint64_t)q3.w << 32) | q3.z;
+    c.k0 = q5.x;
+    c.k1 = q5.y;
+    c.root_begin = ((uint64_t)q5.w << 32) | q5.z;
   } else {
     const TypeDev* t = smem_types + ty;
     const double2 ms = *reinterpret_cast<const double2*>(&t->mu);

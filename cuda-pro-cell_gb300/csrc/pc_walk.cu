@@ -1,0 +1,30 @@
+// Instantiations and launchers of the tree walk (pc_walk.cuh), plain and batched.
+#include "pc_walk.cuh"
+
+namespace pc {
+
+int walk_occupancy(bool batched, int* blocks_per_sm) {
+  auto* k = batched ? k_walk<true> : k_walk<false>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkSmem));
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, kWalkThreads, sizeof(WalkSmem));
+  return (int)e;
+}
+
+uint32_t walk_warps_per_block() { return kWalkWarps; }
+
+int launch_walk(const WalkArgs& w, int blocks, void* stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3((unsigned)kWalkThreads);
+  cfg.dynamicSmemBytes = sizeof(WalkSmem);
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, w.a.btypes ? k_walk<true> : k_walk<false>, w);
+}
+
+}  // namespace pc

@@ -115,6 +115,10 @@ int pc_set_stream(pc_context* ctx, void* stream);
  *   "max_root_chunk"      cap on roots per root-sweep launch (default: from budget)
  *   "grid_blocks"         blocks per launch (default: resident blocks x SMs)
  *   "sweep_config"        compiled sweep configuration 0-7 (default 4; see pc_autotune)
+ *                         With the default configuration and neither max_slice_cells nor
+ *                         max_root_chunk set, a run whose phi caps are at most 31 is one
+ *                         tree walk instead (one cooperative launch, no level buffers;
+ *                         stats count its rounds as sweeps); the sweeps serve the rest.
  *   "driver"              0: one kernel launch per sweep (default); 1: one persistent
  *                         cooperative launch per run
  *   "graph"               1: the persistent driver captures its run in a CUDA graph once
