@@ -75,6 +75,7 @@ struct pc_context {
   // sub-batches of pc_simulate_batch alternate between two live plans)
   Spare spare_rec[kSpares], spare_hist[kSpares];
   Spare spare_tables[kSpares];  // ... and of their small tables (one allocation per plan)
+  Spare spare_map[kSpares];     // ... and of their value maps (the result merge's input)
   std::vector<pc_plan*> live;  // plans created on this context and not yet destroyed
   // pinned host copy of the last count table read back (plan id and run number it holds)
   unsigned long long* stage = nullptr;
@@ -84,8 +85,8 @@ struct pc_context {
   // host threads merge the previous one's
   unsigned long long* stage2 = nullptr;
   size_t stage2_elems = 0;
-  // the device merge of a plan's result: device scratch (value map, type order, merged
-  // counts) and the pinned copy of the merged counts, both grown on demand
+  // the device merge of a plan's result: device scratch (merged counts) and a pinned buffer
+  // (the value map on its way up, the merged counts on their way back), both grown on demand
   void* merge_dev = nullptr;
   size_t merge_dev_bytes = 0;
   unsigned long long* merge_host = nullptr;
@@ -150,6 +151,10 @@ struct pc_plan {
   uint64_t id = 0, run_id = 0;                // identity of the counts in the pinned stage
   pc_context* owner = nullptr;                // receives the large buffers on destroy
   size_t rec_bytes = 0, hist_bytes = 0;
+  // the (bin, generation) -> value map on the device, uploaded by the first result merge
+  void* map_dev = nullptr;
+  size_t map_bytes = 0;
+  bool map_ready = false;
   cudaGraphExec_t graph = nullptr;           // persistent driver: the captured run
   // ... and what it was captured with: the launch's arguments (the persistent sweeps' or the
   // tree walk's), configuration (-1: the tree walk) and grid
@@ -541,6 +546,7 @@ void pc_destroy(pc_context* ctx) {
     pc_cuda_free(ctx->spare_rec[i].p);
     pc_cuda_free(ctx->spare_hist[i].p);
     pc_cuda_free(ctx->spare_tables[i].p);
+    pc_cuda_free(ctx->spare_map[i].p);
   }
   pc_cuda_free(ctx->merge_dev);
   cudaFreeHost(ctx->merge_host);
@@ -1094,50 +1100,108 @@ constexpr size_t kMaxMergeScratch = size_t(256) << 20;
 
 size_t round16(size_t n) { return (n + 15) & ~size_t(15); }
 
+// The device scratch and the pinned buffer of the merge, grown to at least these sizes.
+int ensure_merge(pc_context* ctx, size_t dev_bytes, size_t host_bytes) {
+  if (ctx->merge_dev_bytes < dev_bytes) {
+    pc_cuda_free(ctx->merge_dev);
+    ctx->merge_dev = nullptr;
+    ctx->merge_dev_bytes = 0;
+    PC_CUDA(ctx, pc_cuda_malloc(&ctx->merge_dev, dev_bytes));
+    ctx->merge_dev_bytes = dev_bytes;
+  }
+  if (ctx->merge_host_bytes < host_bytes) {
+    cudaFreeHost(ctx->merge_host);
+    ctx->merge_host = nullptr;
+    ctx->merge_host_bytes = 0;
+    PC_CUDA(ctx, pc_cuda_malloc_host(&ctx->merge_host, host_bytes));
+    ctx->merge_host_bytes = host_bytes;
+  }
+  return PC_OK;
+}
+
+// Bytes of a plan's map: one MergeInstance per instance, their value maps one after another,
+// and (a single instance) its type order.
+size_t merge_map_bytes(const pc_plan* p) {
+  size_t n = round16(p->inst.size() * sizeof(MergeInstance));
+  for (const InstanceHost& I : p->inst) n += round16(I.vidx.size() * sizeof(int32_t));
+  if (!p->batched) n += round16(p->inst[0].sorted_to_file.size() * sizeof(uint32_t));
+  return n;
+}
+
+// The map on the device: it depends on the bins and phi alone, so a plan uploads it with its
+// first merge and keeps it. Staged through the pinned buffer (at least merge_map_bytes).
+int upload_map(pc_context* ctx, pc_plan* p, size_t bytes, uint64_t* uploaded) {
+  *uploaded = 0;
+  if (p->map_ready) return PC_OK;
+  if (!p->map_dev) PC_CUDA(ctx, take_spare(ctx->spare_map, bytes, &p->map_dev, &p->map_bytes));
+  char* const h = reinterpret_cast<char*>(ctx->merge_host);
+  const uint32_t n = (uint32_t)p->inst.size();
+  std::vector<size_t> at(n + 1);
+  at[0] = round16(n * sizeof(MergeInstance));
+  uint64_t values = 0;
+  for (uint32_t i = 0; i < n; ++i) {
+    const InstanceHost& I = p->inst[i];
+    at[i + 1] = at[i] + round16(I.vidx.size() * sizeof(int32_t));
+    MergeInstance m;
+    m.vidx = at[i] / sizeof(int32_t);
+    m.values = values;
+    m.class_begin = I.class_begin;
+    m.bin_begin = I.bin_begin;
+    m.nbins = (uint32_t)I.bin_value.size();
+    m.ntypes = (uint32_t)I.types.size();
+    m.stride = I.vidx_stride;
+    m.gens = I.hist_gens;
+    m.pad = 0;
+    std::memcpy(h + i * sizeof(MergeInstance), &m, sizeof(m));
+    values += I.values.size();
+  }
+  auto copy = [&](uint32_t i) {
+    const InstanceHost& I = p->inst[i];
+    if (!I.vidx.empty()) std::memcpy(h + at[i], I.vidx.data(), I.vidx.size() * sizeof(int32_t));
+  };
+  if (at[n] >= (size_t(1) << 20) && n >= 16) {
+    parallel_for(n, copy, 8);
+  } else {
+    for (uint32_t i = 0; i < n; ++i) copy(i);
+  }
+  if (!p->batched) {
+    const auto& s2f = p->inst[0].sorted_to_file;
+    std::memcpy(h + at[n], s2f.data(), s2f.size() * sizeof(uint32_t));
+  }
+  PC_CUDA(ctx, pc_cuda_copy(p->map_dev, h, bytes, cudaMemcpyHostToDevice, ctx->stream));
+  p->map_ready = true;
+  *uploaded = bytes;
+  return PC_OK;
+}
+
 // The merged histogram of a single-instance plan, merged on the device from the count table
-// the run left there: the value map and type order go up (nbins x generations int32), the
-// merged counts (values x (1 + types) u64) come back, instead of the whole [generation][class]
-// table and a host loop over it. Returns PC_ERR_UNSUPPORTED when the scratch would exceed
-// kMaxMergeScratch.
+// the run left there; the merged counts (values x (1 + types) u64) come back, instead of the
+// whole [generation][class] table and a host loop over it. Returns PC_ERR_UNSUPPORTED when
+// the scratch would exceed kMaxMergeScratch.
 int device_result(pc_context* ctx, pc_plan* p, pc_histogram* out) {
   const InstanceHost& I = p->inst[0];
   const uint32_t nb = (uint32_t)I.bin_value.size(), nt = (uint32_t)I.types.size();
   const uint64_t nv = I.values.size();
-  const size_t vidx_bytes = round16((size_t)nb * I.vidx_stride * sizeof(int32_t));
-  const size_t s2f_bytes = round16((size_t)nt * sizeof(uint32_t));
   const size_t counts = (size_t)nv * (1u + nt) + 2u;  // totals, per_type, error word
-  const size_t need = vidx_bytes + s2f_bytes + counts * sizeof(unsigned long long);
-  if (need > kMaxMergeScratch) return PC_ERR_UNSUPPORTED;
+  const size_t map = merge_map_bytes(p), back = counts * sizeof(unsigned long long);
+  if (map + back > kMaxMergeScratch) return PC_ERR_UNSUPPORTED;
   cudaStream_t st = ctx->stream;
-  if (ctx->merge_dev_bytes < need) {
-    pc_cuda_free(ctx->merge_dev);
-    ctx->merge_dev = nullptr;
-    ctx->merge_dev_bytes = 0;
-    PC_CUDA(ctx, pc_cuda_malloc(&ctx->merge_dev, need));
-    ctx->merge_dev_bytes = need;
-  }
-  if (ctx->merge_host_bytes < counts * sizeof(unsigned long long)) {
-    cudaFreeHost(ctx->merge_host);
-    ctx->merge_host = nullptr;
-    ctx->merge_host_bytes = 0;
-    PC_CUDA(ctx, pc_cuda_malloc_host(&ctx->merge_host, counts * sizeof(unsigned long long)));
-    ctx->merge_host_bytes = counts * sizeof(unsigned long long);
-  }
-  char* base = static_cast<char*>(ctx->merge_dev);
-  int32_t* vidx = reinterpret_cast<int32_t*>(base);
-  uint32_t* s2f = reinterpret_cast<uint32_t*>(base + vidx_bytes);
-  unsigned long long* merged = reinterpret_cast<unsigned long long*>(base + vidx_bytes + s2f_bytes);
+  int rc = ensure_merge(ctx, back, std::max(back, p->map_ready ? size_t(0) : map));
+  uint64_t uploaded = 0;
+  if (rc == PC_OK) rc = upload_map(ctx, p, map, &uploaded);
+  if (rc != PC_OK) return rc;
+  const char* base = static_cast<const char*>(p->map_dev);
+  const int32_t* vidx = reinterpret_cast<const int32_t*>(base + round16(sizeof(MergeInstance)));
+  const uint32_t* s2f = reinterpret_cast<const uint32_t*>(base + round16(sizeof(MergeInstance)) +
+                                                          round16(I.vidx.size() * sizeof(int32_t)));
+  unsigned long long* merged = static_cast<unsigned long long*>(ctx->merge_dev);
   unsigned long long* totals = merged;
   unsigned long long* per_type = merged + nv;
   uint32_t* error = reinterpret_cast<uint32_t*>(merged + nv * (1u + nt));
-  if (nb)
-    PC_CUDA(ctx, pc_cuda_copy(vidx, I.vidx.data(), (size_t)nb * I.vidx_stride * sizeof(int32_t),
-                              cudaMemcpyHostToDevice, st));
-  PC_CUDA(ctx, pc_cuda_copy(s2f, I.sorted_to_file.data(), (size_t)nt * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-  PC_CUDA(ctx, pc_cuda_memset(merged, 0, counts * sizeof(unsigned long long), st));
+  PC_CUDA(ctx, pc_cuda_memset(merged, 0, back, st));
   PC_CUDA(ctx, PC_LAUNCH(launch_merge_counts(p->hist_dev, p->nclass, I.class_begin, I.hist_gens, nb, nt, vidx,
                                              I.vidx_stride, s2f, totals, per_type, error, st)));
-  PC_CUDA(ctx, pc_cuda_copy(ctx->merge_host, merged, counts * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  PC_CUDA(ctx, pc_cuda_copy(ctx->merge_host, merged, back, cudaMemcpyDeviceToHost, st));
   PC_CUDA(ctx, pc_cuda_sync(st));
   const unsigned long long* hm = ctx->merge_host;
   if (static_cast<uint32_t>(hm[nv * (1u + nt)]) & 1u)
@@ -1159,8 +1223,31 @@ int device_result(pc_context* ctx, pc_plan* p, pc_histogram* out) {
   uint64_t leaves = 0;
   for (uint64_t v = 0; v < nv; ++v) leaves += hm[v];
   out->stats.leaves = leaves;
-  out->stats.h2d_bytes = (uint64_t)nb * I.vidx_stride * sizeof(int32_t) + (uint64_t)nt * sizeof(uint32_t);
-  out->stats.d2h_bytes = counts * sizeof(unsigned long long);
+  out->stats.h2d_bytes = uploaded;
+  out->stats.d2h_bytes = back;
+  return PC_OK;
+}
+
+// The merged totals of every instance of a batch, merged on the device: the totals come back
+// (values u64) instead of the whole count table. PC_ERR_UNSUPPORTED as device_result.
+int device_totals(pc_context* ctx, pc_plan* p, uint64_t nv, uint64_t* out) {
+  const size_t map = merge_map_bytes(p), back = (nv + 2u) * sizeof(unsigned long long);
+  if (map + back > kMaxMergeScratch) return PC_ERR_UNSUPPORTED;
+  cudaStream_t st = ctx->stream;
+  int rc = ensure_merge(ctx, back, std::max(back, p->map_ready ? size_t(0) : map));
+  uint64_t uploaded = 0;
+  if (rc == PC_OK) rc = upload_map(ctx, p, map, &uploaded);
+  if (rc != PC_OK) return rc;
+  unsigned long long* totals = static_cast<unsigned long long*>(ctx->merge_dev);
+  uint32_t* error = reinterpret_cast<uint32_t*>(totals + nv);
+  PC_CUDA(ctx, pc_cuda_memset(totals, 0, back, st));
+  PC_CUDA(ctx, PC_LAUNCH(launch_merge_totals(p->hist_dev, p->nclass, p->map_dev, (uint32_t)p->inst.size(),
+                                             p->hist_gens, p->nbins, p->bin_inst_dev, totals, error, st)));
+  PC_CUDA(ctx, pc_cuda_copy(ctx->merge_host, totals, back, cudaMemcpyDeviceToHost, st));
+  PC_CUDA(ctx, pc_cuda_sync(st));
+  if (static_cast<uint32_t>(ctx->merge_host[nv]) & 1u)
+    return fail(ctx, PC_ERR_CUDA, "internal: leaf counted outside the output value set");
+  std::memcpy(out, ctx->merge_host, nv * sizeof(uint64_t));
   return PC_OK;
 }
 
@@ -1320,10 +1407,12 @@ void pc_plan_destroy(pc_plan* p) {
     give_spare(ctx->spare_tables, p->tables_dev, p->tables_bytes);
     give_spare(ctx->spare_rec, p->root_rec_dev, p->rec_bytes);
     give_spare(ctx->spare_hist, p->hist_dev, p->hist_bytes);
+    give_spare(ctx->spare_map, p->map_dev, p->map_bytes);
   } else {
     pc_cuda_free(p->tables_dev);
     pc_cuda_free(p->root_rec_dev);
     pc_cuda_free(p->hist_dev);
+    pc_cuda_free(p->map_dev);
   }
   delete p;
 }
@@ -2111,6 +2200,11 @@ int pc_batch_totals(pc_context* ctx, pc_batch* b, uint64_t* out, uint64_t capaci
   if (!out) return PC_OK;
   if (capacity < off[n]) return fail(ctx, PC_ERR_INVALID, "totals buffer too small");
   if (!b->ran) return fail(ctx, PC_ERR_INVALID, "batch has not run");
+  PC_CUDA(ctx, cudaSetDevice(ctx->device));
+  if (ctx->opt_device_merge && b->nbins != 0) {
+    const int rd = device_totals(ctx, b, off[n], out);
+    if (rd != PC_ERR_UNSUPPORTED) return rd;
+  }
   const unsigned long long* h = nullptr;
   const int rc = stage_table(ctx, b, &h);
   if (rc != PC_OK) return rc;

@@ -235,6 +235,17 @@ int occupancy_blocks_per_sm(int* root_blocks, int* divide_blocks);
 int launch_merge_counts(const unsigned long long* hist, uint64_t nclass, uint64_t class_begin, uint32_t hist_gens,
                         uint32_t nb, uint32_t nt, const int32_t* vidx, uint32_t vidx_stride, const uint32_t* s2f,
                         unsigned long long* totals, unsigned long long* per_type, uint32_t* error, void* stream);
+// The merged totals of a batch: map = [ninst] MergeInstance, then their value maps; thread
+// (g, b) adds the counts of bin b of the batch at generation g to its value's total.
+struct MergeInstance {
+  uint64_t vidx;         // first int32 of its value map, from the start of the map
+  uint64_t values;       // its first total
+  uint64_t class_begin;  // its first histogram class
+  uint32_t bin_begin, nbins, ntypes, stride, gens, pad;
+};
+int launch_merge_totals(const unsigned long long* hist, uint64_t nclass, const void* map, uint32_t ninst,
+                        uint32_t hist_gens, uint32_t nbins, const uint32_t* bin_inst, unsigned long long* totals,
+                        uint32_t* error, void* stream);
 // Throughput probe (roofline denominators): kind 0 FP64 FMA, 1 FP32 FMA, 2 INT32 multiply-add;
 // each of the blocks x 256 threads runs iters x 8 operations.
 int launch_peak_probe(int kind, uint32_t iters, int blocks, double* sink, void* stream);
