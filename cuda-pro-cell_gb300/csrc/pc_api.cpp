@@ -20,8 +20,9 @@
 #include <cstring>
 #include <atomic>
 #include <chrono>
+#include <condition_variable>
 #include <map>
-#include <new>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -397,8 +398,96 @@ void give_spare(Spare* spare, void* buf, size_t bytes) {
   spare[slot].bytes = bytes;
 }
 
+// Host worker threads, started on first use and kept for the process (starting 15 threads
+// costs 0.4 ms on this machine's cores, several times the work of a small batch's merge). Any
+// number of calling threads may post jobs. A caller works on its own job and returns when it
+// is done and no worker still runs it, so a job ends even if no worker ever takes it (no
+// thread could be started, or a forked child, which has none).
+class Workers {
+ public:
+  static Workers& get() {
+    static Workers* w = new Workers();  // never destroyed: its threads may outlive main
+    return *w;
+  }
+  // f(i) for i in [0, n), on at most `helpers` workers and the calling thread. The first
+  // exception of any of them is rethrown here.
+  template <class F>
+  void run(uint32_t n, unsigned helpers, F&& f) {
+    Job job;
+    job.n = n;
+    job.wanted = helpers;
+    job.call = [](void* p, uint32_t i) { (*static_cast<std::remove_reference_t<F>*>(p))(i); };
+    job.arg = const_cast<void*>(static_cast<const void*>(&f));
+    {
+      std::lock_guard<std::mutex> lock(m_);
+      while (threads_ < std::min(helpers, max_)) {
+        try {
+          std::thread([this] { serve(); }).detach();
+          ++threads_;
+        } catch (...) {
+          break;
+        }
+      }
+      jobs_.push_back(&job);
+    }
+    ready_.notify_all();
+    work(job);
+    std::unique_lock<std::mutex> lock(m_);
+    jobs_.erase(std::remove(jobs_.begin(), jobs_.end(), &job), jobs_.end());
+    job.left.wait(lock, [&] { return job.active == 0; });
+    if (job.error) std::rethrow_exception(job.error);
+  }
+
+ private:
+  struct Job {
+    uint32_t n = 0;
+    unsigned wanted = 0, active = 0;  // workers still welcome, workers on it (under m_)
+    void (*call)(void*, uint32_t) = nullptr;
+    void* arg = nullptr;
+    std::atomic<uint32_t> next{0};
+    std::mutex error_m;
+    std::exception_ptr error;
+    std::condition_variable left;
+  };
+  static void work(Job& job) {
+    try {
+      for (uint32_t i; (i = job.next.fetch_add(1)) < job.n;) job.call(job.arg, i);
+    } catch (...) {
+      job.next = job.n;
+      std::lock_guard<std::mutex> lock(job.error_m);
+      if (!job.error) job.error = std::current_exception();
+    }
+  }
+  void serve() {
+    std::unique_lock<std::mutex> lock(m_);
+    for (;;) {
+      Job* job = nullptr;
+      for (Job* j : jobs_)
+        if (j->wanted != 0 && j->next.load() < j->n) {
+          job = j;
+          break;
+        }
+      if (!job) {
+        ready_.wait(lock);
+        continue;
+      }
+      --job->wanted;
+      ++job->active;
+      lock.unlock();
+      work(*job);
+      lock.lock();
+      if (--job->active == 0) job->left.notify_all();
+    }
+  }
+  const unsigned max_ = std::min(63u, std::max(1u, std::thread::hardware_concurrency()));
+  std::mutex m_;
+  std::condition_variable ready_;
+  std::vector<Job*> jobs_;
+  unsigned threads_ = 0;
+};
+
 // f(i) for i in [0, n) on up to `threads` host threads (0 = all cores), the calling thread
-// among them. A thread that cannot be started leaves its share to the others.
+// among them.
 template <class F>
 void parallel_for(uint32_t n, F&& f, unsigned threads = 0) {
   unsigned nt = threads ? threads : std::max(1u, std::thread::hardware_concurrency());
@@ -407,21 +496,114 @@ void parallel_for(uint32_t n, F&& f, unsigned threads = 0) {
     for (uint32_t i = 0; i < n; ++i) f(i);
     return;
   }
-  std::atomic<uint32_t> next{0};
-  auto work = [&]() {
-    for (uint32_t i; (i = next.fetch_add(1)) < n;) f(i);
+  Workers::get().run(n, nt - 1, f);
+}
+
+// The arrays of result histograms. Large ones come from fresh pages that each cost a fault on
+// first use (a third of the time of reading a 7 MB result), so freed ones are kept for the next
+// results: at most kKept bytes in the process, any thread may allocate or free.
+class ResultMemory {
+ public:
+  static ResultMemory& get() {
+    static ResultMemory* r = new ResultMemory();
+    return *r;
+  }
+  void* allocate(size_t bytes) {
+    if (bytes < kSmall) return std::malloc(std::max<size_t>(1, bytes));
+    std::lock_guard<std::mutex> lock(m_);
+    const auto it = kept_.lower_bound(bytes);
+    if (it != kept_.end() && it->first <= 2 * bytes) {
+      void* p = it->second;
+      const size_t size = it->first;
+      kept_.erase(it);
+      kept_bytes_ -= size;
+      out_[p] = size;
+      return p;
+    }
+    void* p = std::malloc(bytes);
+    if (p) out_[p] = bytes;
+    return p;
+  }
+  // Pinned memory for the device to write a result's counts into directly (copying 7 MB out of
+  // a staging buffer takes 0.35 ms): nullptr when none of kBlocks is free or large enough. Its
+  // `refs` arrays are handed out with give_pinned and released one by one.
+  struct Block {
+    void* p = nullptr;
+    size_t bytes = 0;
+    int refs = 0;
   };
-  std::vector<std::thread> pool;
-  pool.reserve(nt - 1);
-  for (unsigned t = 0; t + 1 < nt; ++t) {
-    try {
-      pool.emplace_back(work);
-    } catch (...) {
-      break;
+  static constexpr size_t kPinnedFrom = size_t(1) << 20, kPinnedMost = size_t(64) << 20;
+  Block* take_pinned(size_t bytes) {
+    if (bytes < kPinnedFrom || bytes > kPinnedMost) return nullptr;
+    std::lock_guard<std::mutex> lock(m_);
+    Block* grow = nullptr;
+    for (Block& b : blocks_) {
+      if (b.refs != 0) continue;
+      if (b.bytes >= bytes) {
+        b.refs = 1;
+        return &b;
+      }
+      grow = &b;
+    }
+    if (!grow) return nullptr;
+    if (grow->p) cudaFreeHost(grow->p);
+    *grow = Block();
+    if (pc_cuda_malloc_host(&grow->p, bytes) != cudaSuccess) {
+      (void)cudaGetLastError();
+      grow->p = nullptr;
+      return nullptr;
+    }
+    grow->bytes = bytes;
+    grow->refs = 1;
+    return grow;
+  }
+  void give_pinned(Block* b, std::initializer_list<void*> arrays) {
+    std::lock_guard<std::mutex> lock(m_);
+    b->refs = 0;
+    for (void* a : arrays) {
+      pinned_[a] = b;
+      ++b->refs;
     }
   }
-  work();
-  for (auto& th : pool) th.join();
+  void release(void* p) {
+    if (!p) return;
+    std::unique_lock<std::mutex> lock(m_);
+    const auto pin = pinned_.find(p);
+    if (pin != pinned_.end()) {
+      --pin->second->refs;
+      pinned_.erase(pin);
+      return;
+    }
+    const auto it = out_.find(p);
+    if (it == out_.end()) {
+      lock.unlock();
+      std::free(p);
+      return;
+    }
+    const size_t size = it->second;
+    out_.erase(it);
+    if (kept_bytes_ + size <= kKept) {
+      kept_.emplace(size, p);
+      kept_bytes_ += size;
+      return;
+    }
+    lock.unlock();
+    std::free(p);
+  }
+
+ private:
+  static constexpr size_t kSmall = size_t(64) << 10, kKept = size_t(64) << 20;
+  std::mutex m_;
+  std::multimap<size_t, void*> kept_;
+  std::map<void*, size_t> out_;
+  size_t kept_bytes_ = 0;
+  static constexpr int kBlocks = 3;
+  Block blocks_[kBlocks];
+  std::map<void*, Block*> pinned_;
+};
+template <class T>
+T* result_array(uint64_t n) {
+  return static_cast<T*>(ResultMemory::get().allocate(n * sizeof(T)));
 }
 
 uint32_t bits_for(uint64_t n) {  // bits needed for values in [0, n)
@@ -1015,7 +1197,7 @@ int finalize_plan(pc_context* ctx, pc_plan* p) {
 // tables. Touches no context state and makes no CUDA call (runs on any thread); messages
 // number the instances from `first`.
 int prepare_batch(const pc_instance* instances, uint32_t n, uint32_t first, uint64_t max_root_chunk,
-                  pc_batch** out, PlanTables& t, std::string& msg) {
+                  pc_batch** out, PlanTables& t, std::string& msg, bool with_values = true) {
   *out = nullptr;
   if (n == 0) return msg = "a batch needs at least one instance", PC_ERR_INVALID;
   pc_batch* b = new (std::nothrow) pc_batch();
@@ -1028,7 +1210,8 @@ int prepare_batch(const pc_instance* instances, uint32_t n, uint32_t first, uint
   std::vector<std::string> msgs(n);
   parallel_for(n, [&](uint32_t i) {
     const pc_instance& x = instances[i];
-    codes[i] = prepare_instance(x.bins, x.n_bins, x.types, x.n_types, x.t_max, x.phi, x.seed, b->inst[i], msgs[i]);
+    codes[i] = prepare_instance(x.bins, x.n_bins, x.types, x.n_types, x.t_max, x.phi, x.seed, b->inst[i], msgs[i],
+                                with_values);
   });
   int rc = PC_OK;
   for (uint32_t i = 0; i < n && rc == PC_OK; ++i)
@@ -1063,15 +1246,19 @@ int instance_result(const pc_plan* p, const InstanceHost& I, const unsigned long
   const uint64_t nv = I.values.size();
   out->n_values = nv;
   out->n_types = nt;
-  out->values = (double*)std::malloc(std::max<uint64_t>(1, nv) * sizeof(double));
-  out->totals = (uint64_t*)std::calloc(std::max<uint64_t>(1, nv), sizeof(uint64_t));
-  out->per_type = (uint64_t*)std::calloc(std::max<uint64_t>(1, nv * nt), sizeof(uint64_t));
+  out->values = result_array<double>(nv);
+  out->totals = result_array<uint64_t>(nv);
+  out->per_type = result_array<uint64_t>(nv * nt);
   if (!out->values || !out->totals || !out->per_type) {
     pc_histogram_free(out);
     *msg = "host allocation";
     return PC_ERR_NOMEM;
   }
-  if (nv) std::memcpy(out->values, I.values.data(), nv * sizeof(double));
+  if (nv) {
+    std::memcpy(out->values, I.values.data(), nv * sizeof(double));
+    std::memset(out->totals, 0, nv * sizeof(uint64_t));
+    std::memset(out->per_type, 0, nv * nt * sizeof(uint64_t));
+  }
   uint64_t leaves = 0;
   for (uint32_t g = 0; g < I.hist_gens; ++g)
     for (uint32_t b = 0; b < nb; ++b) {
@@ -1201,22 +1388,43 @@ int device_result(pc_context* ctx, pc_plan* p, pc_histogram* out) {
   PC_CUDA(ctx, pc_cuda_memset(merged, 0, back, st));
   PC_CUDA(ctx, PC_LAUNCH(launch_merge_counts(p->hist_dev, p->nclass, I.class_begin, I.hist_gens, nb, nt, vidx,
                                              I.vidx_stride, s2f, totals, per_type, error, st)));
-  PC_CUDA(ctx, pc_cuda_copy(ctx->merge_host, merged, back, cudaMemcpyDeviceToHost, st));
-  PC_CUDA(ctx, pc_cuda_sync(st));
-  const unsigned long long* hm = ctx->merge_host;
-  if (static_cast<uint32_t>(hm[nv * (1u + nt)]) & 1u)
+  // into memory that is handed out as it is, where there is some, else through the stage
+  struct Pinned {
+    ResultMemory::Block* b;
+    ~Pinned() {
+      if (b) ResultMemory::get().give_pinned(b, {});
+    }
+  } pinned{ResultMemory::get().take_pinned(back)};
+  unsigned long long* const hm = pinned.b ? static_cast<unsigned long long*>(pinned.b->p) : ctx->merge_host;
+  PC_CUDA(ctx, pc_cuda_copy(hm, merged, back, cudaMemcpyDeviceToHost, st));
+  out->values = result_array<double>(nv);  // copied while the counts come back
+  if (nv && out->values) std::memcpy(out->values, I.values.data(), nv * sizeof(double));
+  const cudaError_t es = pc_cuda_sync(st);
+  if (es != cudaSuccess) {
+    cudaStreamSynchronize(st);  // nothing may still write to the result's memory
+    pc_histogram_free(out);
+  }
+  PC_CUDA(ctx, es);
+  if (static_cast<uint32_t>(hm[nv * (1u + nt)]) & 1u) {
+    pc_histogram_free(out);
     return fail(ctx, PC_ERR_CUDA, "internal: leaf counted outside the output value set");
+  }
   out->n_values = nv;
   out->n_types = nt;
-  out->values = (double*)std::malloc(std::max<uint64_t>(1, nv) * sizeof(double));
-  out->totals = (uint64_t*)std::malloc(std::max<uint64_t>(1, nv) * sizeof(uint64_t));
-  out->per_type = (uint64_t*)std::malloc(std::max<uint64_t>(1, nv * nt) * sizeof(uint64_t));
+  if (pinned.b) {
+    out->totals = reinterpret_cast<uint64_t*>(hm);
+    out->per_type = reinterpret_cast<uint64_t*>(hm + nv);
+    ResultMemory::get().give_pinned(pinned.b, {out->totals, out->per_type});
+    pinned.b = nullptr;
+  } else {
+    out->totals = result_array<uint64_t>(nv);
+    out->per_type = result_array<uint64_t>(nv * nt);
+  }
   if (!out->values || !out->totals || !out->per_type) {
     pc_histogram_free(out);
     return fail(ctx, PC_ERR_NOMEM, "host allocation");
   }
-  if (nv) {
-    std::memcpy(out->values, I.values.data(), nv * sizeof(double));
+  if (nv && out->totals != reinterpret_cast<uint64_t*>(hm)) {
     std::memcpy(out->totals, hm, nv * sizeof(uint64_t));
     std::memcpy(out->per_type, hm + nv, nv * nt * sizeof(uint64_t));
   }
@@ -2019,9 +2227,10 @@ int pc_plan_result(pc_context* ctx, pc_plan* p, pc_histogram* out) {
 
 void pc_histogram_free(pc_histogram* h) {
   if (!h) return;
-  std::free(h->values);
-  std::free(h->totals);
-  std::free(h->per_type);
+  ResultMemory& r = ResultMemory::get();
+  r.release(h->values);
+  r.release(h->totals);
+  r.release(h->per_type);
   h->values = nullptr;
   h->totals = nullptr;
   h->per_type = nullptr;
@@ -2275,7 +2484,7 @@ int pc_simulate_batch(pc_context* ctx, const pc_instance* instances, uint32_t n_
   auto prepare_part = [&](uint32_t part, Prepared& pr) {
     try {
       pr.rc = prepare_batch(instances + first_of(part), first_of(part + 1) - first_of(part), first_of(part),
-                            max_root_chunk, &pr.b, pr.t, pr.msg);
+                            max_root_chunk, &pr.b, pr.t, pr.msg, part != 0);
     } catch (...) {
       pr.rc = PC_ERR_NOMEM;
       pr.msg = "host allocation";
@@ -2324,7 +2533,27 @@ int pc_simulate_batch(pc_context* ctx, const pc_instance* instances, uint32_t n_
         prepare_part(part + 1u, nxt);  // no thread to overlap with: prepare here
       }
     }
+    // the first part's output value sets, which only its merge reads, are built during its run
+    // (the other parts' while an earlier one runs)
+    bool built = part != 0;
+    Joined values;
+    auto build = [b, &built] {
+      try {
+        parallel_for((uint32_t)b->inst.size(), [b](uint32_t i) { build_value_set(b->inst[i]); });
+        built = true;
+      } catch (...) {
+      }
+    };
+    if (rc == PC_OK && !built) {
+      try {
+        values.th = std::thread(build);
+      } catch (...) {  // no thread: build them here
+        build();
+      }
+    }
     if (rc == PC_OK) rc = pc_batch_run(ctx, b);
+    if (values.th.joinable()) values.th.join();
+    if (rc == PC_OK && !built) rc = fail(ctx, PC_ERR_NOMEM, "host allocation");
     const unsigned long long* h = nullptr;
     // every part but the last has its count table copied back while the next part runs;
     // its merge waits for that copy

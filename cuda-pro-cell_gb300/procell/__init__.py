@@ -59,12 +59,9 @@ class Plan:
         return {k: getattr(st, k) for k, _ in _lib.Stats._fields_}
 
     def result(self) -> Result:
-        h = _lib.Histogram()
-        self.engine._check(self.engine.L.pc_plan_result(self.engine.ctx, self.handle, ctypes.byref(h)))
-        try:
-            return Result(*_lib.histogram_to_numpy(h))
-        finally:
-            self.engine.L.pc_histogram_free(ctypes.byref(h))
+        h = (_lib.Histogram * 1)()
+        self.engine._check(self.engine.L.pc_plan_result(self.engine.ctx, self.handle, h))
+        return Result(*_lib.histograms_to_numpy(h, 1)[0])
 
     def raw_counts(self) -> np.ndarray:
         L, n = self.engine.L, ctypes.c_uint64()
@@ -92,9 +89,8 @@ class Plan:
 def instance_array(instances):
     """A pc_instance array of (bins, types, t_max, phi, seed) tuples or dicts, and the numpy
     arrays it points into (keep them alive while the array is used)."""
-    keep = []
-    arr = (_lib.Instance * max(1, len(instances)))()
-    for i, inst in enumerate(instances):
+    keep, rows = [], []
+    for inst in instances:
         if isinstance(inst, dict):
             bins, types, t_max = inst["bins"], inst["types"], inst["t_max"]
             phi, seed = inst.get("phi"), inst.get("seed", 0)
@@ -102,14 +98,11 @@ def instance_array(instances):
             bins, types, t_max, phi, seed = inst
         b, t = _lib.bins_numpy(bins), _lib.types_numpy(types)
         keep += [b, t]
-        arr[i].bins = b.ctypes.data_as(ctypes.POINTER(_lib.Bin))
-        arr[i].n_bins = len(b)
-        arr[i].types = t.ctypes.data_as(ctypes.POINTER(_lib.CellType))
-        arr[i].n_types = len(t)
-        arr[i].reserved = 0
-        arr[i].t_max = float(t_max)
-        arr[i].phi = 0.0 if phi is None else float(phi)
-        arr[i].seed = int(seed)
+        rows.append((b.__array_interface__["data"][0], len(b), t.__array_interface__["data"][0], len(t), 0, float(t_max),
+                     0.0 if phi is None else float(phi), int(seed) & 0xFFFFFFFFFFFFFFFF))
+    arr = (_lib.Instance * max(1, len(instances)))()
+    if rows:
+        np.frombuffer(arr, _lib.INSTANCE_DTYPE, len(rows))[:] = rows
     return arr, keep
 
 
@@ -135,12 +128,9 @@ class Batch:
         return {k: getattr(st, k) for k, _ in _lib.Stats._fields_}
 
     def result(self, i: int) -> Result:
-        h = _lib.Histogram()
-        self.engine._check(self.engine.L.pc_batch_result(self.engine.ctx, self.handle, int(i), ctypes.byref(h)))
-        try:
-            return Result(*_lib.histogram_to_numpy(h))
-        finally:
-            self.engine.L.pc_histogram_free(ctypes.byref(h))
+        h = (_lib.Histogram * 1)()
+        self.engine._check(self.engine.L.pc_batch_result(self.engine.ctx, self.handle, int(i), h))
+        return Result(*_lib.histograms_to_numpy(h, 1)[0])
 
     def set_types(self, types):
         """New cell types for every instance: a TYPE_DTYPE array (or rows of (ratio, mean,
@@ -226,35 +216,24 @@ class Engine:
         n = len(instances)
         hs = (_lib.Histogram * max(1, n))()
         self._check(self.L.pc_simulate_batch(self.ctx, arr, n, hs))
-        out = []
-        try:
-            for i in range(n):
-                out.append(Result(*_lib.histogram_to_numpy(hs[i])))
-        finally:
-            for i in range(n):
-                self.L.pc_histogram_free(ctypes.byref(hs[i]))
         del keep
-        return out
+        return [Result(*r) for r in _lib.histograms_to_numpy(hs, n)]
 
     def simulate(self, bins, types, t_max, phi=None, seed=0, root_begin=None, root_end=None) -> Result:
         """pc_simulate (pc_simulate_shard for a range of initial cells): one input's merged
         histogram, host arrays in and out, in one library call."""
         b, t = _lib.bins_numpy(bins), _lib.types_numpy(types)
-        h = _lib.Histogram()
+        h = (_lib.Histogram * 1)()
         args = (self.ctx, b.ctypes.data_as(ctypes.POINTER(_lib.Bin)), len(b),
                 t.ctypes.data_as(ctypes.POINTER(_lib.CellType)), len(t), float(t_max),
                 0.0 if phi is None else float(phi), int(seed))
         if root_begin is not None or root_end is not None:
             total = int(b["frequency"].sum())
-            rc = self.L.pc_simulate_shard(*args, int(root_begin or 0), total if root_end is None else int(root_end),
-                                          ctypes.byref(h))
+            rc = self.L.pc_simulate_shard(*args, int(root_begin or 0), total if root_end is None else int(root_end), h)
         else:
-            rc = self.L.pc_simulate(*args, ctypes.byref(h))
-        try:
-            self._check(rc)
-            return Result(*_lib.histogram_to_numpy(h))
-        finally:
-            self.L.pc_histogram_free(ctypes.byref(h))
+            rc = self.L.pc_simulate(*args, h)
+        self._check(rc)
+        return Result(*_lib.histograms_to_numpy(h, 1)[0])
 
     def get_option(self, name: str) -> float:
         v = ctypes.c_double()

@@ -169,6 +169,7 @@ def types_array(types):
 
 
 def histogram_to_numpy(h: Histogram):
+    """Copies of a histogram's arrays (the caller still frees it)."""
     nv, nt = int(h.n_values), int(h.n_types)
     values = np.ctypeslib.as_array(h.values, shape=(max(1, nv),))[:nv].copy()
     totals = np.ctypeslib.as_array(h.totals, shape=(max(1, nv),))[:nv].copy()
@@ -178,6 +179,52 @@ def histogram_to_numpy(h: Histogram):
     return values, totals.astype(np.uint64, copy=False), per.astype(np.uint64, copy=False), stats
 
 
+HISTOGRAM_DTYPE = np.dtype({
+    "names": ["n_values", "n_types", "values", "totals", "per_type"],
+    "formats": ["<u8", "<u4", "<u8", "<u8", "<u8"],
+    "offsets": [getattr(Histogram, k).offset for k in ("n_values", "n_types", "values", "totals", "per_type")],
+    "itemsize": ctypes.sizeof(Histogram)})
+_STATS = [k for k, _ in Stats._fields_]
+
+
+class _Owner:
+    """A histogram filled by the library, freed when the last array on its memory is gone."""
+    __slots__ = ("h",)
+
+    def __init__(self, h):
+        self.h = h
+
+    def __del__(self):
+        try:
+            _lib.pc_histogram_free(ctypes.byref(self.h))
+        except Exception:  # interpreter shutdown
+            pass
+
+
+class _View:
+    __slots__ = ("__array_interface__", "owner")
+
+    def __init__(self, owner, address, shape, typestr):
+        self.owner = owner
+        self.__array_interface__ = {"data": (address, False), "shape": shape, "typestr": typestr, "version": 3}
+
+
+def histograms_to_numpy(hs, n):
+    """(values, totals, per_type, stats) of each of the n histograms of the ctypes array `hs`,
+    arrays on the library's own memory, which they keep alive (no copy)."""
+    out = []
+    for i, (nv, nt, values, totals, per_type) in enumerate(np.frombuffer(hs, HISTOGRAM_DTYPE, n).tolist()):
+        h = hs[i]
+        own = _Owner(h)
+        st = h.stats
+        out.append((np.asarray(_View(own, values, (nv,), "<f8")), np.asarray(_View(own, totals, (nv,), "<u8")),
+                    np.asarray(_View(own, per_type, (nv, nt), "<u8")), {k: getattr(st, k) for k in _STATS}))
+    return out
+
+
+INSTANCE_DTYPE = np.dtype([("bins", "<u8"), ("n_bins", "<u8"), ("types", "<u8"), ("n_types", "<u4"), ("reserved", "<u4"),
+                           ("t_max", "<f8"), ("phi", "<f8"), ("seed", "<u8")])
+assert INSTANCE_DTYPE.itemsize == ctypes.sizeof(Instance)
 BIN_DTYPE = np.dtype([("value", "<f8"), ("frequency", "<u8")])
 TYPE_DTYPE = np.dtype([("ratio", "<f8"), ("mean", "<f8"), ("sd", "<f8")])
 
@@ -198,6 +245,8 @@ def bins_numpy(bins) -> np.ndarray:
 
 
 def types_numpy(types) -> np.ndarray:
+    if type(types) is list and all(type(t) is tuple and len(t) == 3 for t in types):
+        return np.array(types, TYPE_DTYPE)
     out = np.empty(len(types), TYPE_DTYPE)
     for i, (r, m, sd) in enumerate(types):
         out[i] = (float(r), float(m), float(sd))
