@@ -2808,7 +2808,7 @@ struct pc_smooth {
   double* e_raw_dev = nullptr;   // [cand_cap][ntypes][nbins][rows]
   double* part_dev = nullptr;    // [cand_cap][nbins][ntypes * 3]
   uint32_t cand_cap = 0;
-  double* jac_raw_dev = nullptr;  // [jac_cap][nbins][rows][ntypes * 3], allocated on first use
+  double* jac_raw_dev = nullptr;  // [jac_cap][nbins][rows][ntypes * 3] and [values], allocated on first use
   uint32_t jac_cap = 0;
   uint32_t* order_dev = nullptr;  // [ntypes][order_cap]: candidates by mean, per type
   uint32_t order_cap = 0;
@@ -2877,7 +2877,7 @@ int jacobian_scratch(pc_context* ctx, pc_smooth* s, uint32_t ncand) {
   s->jac_raw_dev = nullptr;
   s->jac_cap = 0;
   const size_t nb = std::max<size_t>(1, s->I.bin_value.size());
-  PC_CUDA(ctx, pc_cuda_malloc(&s->jac_raw_dev, (size_t)ncand * nb * s->rows * s->ntypes * 3 * sizeof(double)));
+  PC_CUDA(ctx, pc_cuda_malloc(&s->jac_raw_dev, ((size_t)ncand * nb * s->rows * s->ntypes * 3 + s->I.values.size()) * sizeof(double)));
   s->jac_cap = ncand;
   return PC_OK;
 }

@@ -41,6 +41,9 @@
 // and the types are added in a fixed order by the merge, so results are deterministic.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "pc_engine.h"
 
 namespace pc {
@@ -50,16 +53,15 @@ namespace {
 constexpr int kThreads = 128;
 constexpr uint32_t kBudget = 1u << 16;
 // Resident blocks per SM the lineage-walk kernels are compiled for (registers per thread =
-// 65536 / (128 x this)); compile-time tuning, results do not depend on it. Measured on the
-// calibration input with the draws made in every pass: 5 blocks (96 registers) forward
-// 1.91 ms, adjoint 2.62 ms; 6 (80 registers) 1.75 / 2.45 ms; 8 (64 registers) 3.04 / 2.45 ms:
-// 6 for those kernels. With the plan's draws kept in device memory they need fewer registers:
-// 6 blocks forward 1.170, adjoint 1.321, Jacobian 1.380 ms; 7 (72 registers, no spills) 1.115
-// / 1.267 / 1.301 ms; 8 (64 registers) 1.066 / 1.213 ms, the Jacobian held at 7 by its shared
-// memory (4 floats per generation row and thread).
+// 65536 / (128 x this)); compile-time tuning, results do not depend on it. Drawing in every
+// pass (calibration input, one walk per lane): 5 blocks forward 1.91, adjoint 2.62 ms; 6 1.75 /
+// 2.45; 8 3.04 / 2.45. Kept draws, two walks per lane, 256 candidates: forward 8 blocks 0.782,
+// 7 0.778, 6 0.831, 5 0.824 ms; Jacobian 7 0.916, 6 0.909, 5 0.912, 4 0.947; adjoint 6 (all its
+// shared memory allows) 0.979, 5 1.048.
 constexpr int kBlocksDrawn = 6;
-constexpr int kBlocksKept = 8;
-constexpr int kBlocksKeptJacobian = 7;
+constexpr int kBlocksKept = 7;
+constexpr int kBlocksKeptJacobian = 6;
+constexpr int kBlocksKeptAdjoint = 6;
 
 __device__ __forceinline__ double f32_to_f64_bits(float z) {
   const uint32_t f = __float_as_uint(z);
@@ -278,22 +280,30 @@ __device__ __forceinline__ LineageU lineage_u(double u) {
 // zbuf[j * 32 + lane] and the block's u tables: read back from the plan's lineage tables
 // (Kept), or drawn here when the plan keeps none. The kernels are instantiated for both, so
 // neither path's code (the draw's FP64 set-up in particular) runs predicated in the other.
-template <bool Kept>
-__device__ __forceinline__ void stage_lineage(const SmoothArgs& A, const ZigTables& Z, uint64_t r0, uint64_t i,
+__device__ __forceinline__ void stage_kept(const SmoothArgs& A, uint64_t r0, uint64_t i, uint32_t steps, float* zlane,
+                                           double* u_age, float* u_one, float* u_one_lo) {
+  const uint64_t L = r0 * A.paths + i;
+  const float4* zr = reinterpret_cast<const float4*>(A.lin_z + L * A.zrow);
+  for (uint32_t j = 0; j < steps; j += 4u) {
+    const float4 q = __ldg(zr + j / 4u);
+    zlane[j * 32u] = q.x;
+    if (j + 1u < steps) zlane[(j + 1u) * 32u] = q.y;
+    if (j + 2u < steps) zlane[(j + 2u) * 32u] = q.z;
+    if (j + 3u < steps) zlane[(j + 3u) * 32u] = q.w;
+  }
+  const LineageU lu = A.lin_u[L];
+  *u_age = lu.u;
+  *u_one = lu.hi;
+  *u_one_lo = lu.lo;
+}
+template <bool Kept, class Tables>
+__device__ __forceinline__ void stage_lineage(const SmoothArgs& A, const Tables& Z, uint64_t r0, uint64_t i,
                                               uint32_t steps, float* zlane, double* u_age, float* u_one,
                                               float* u_one_lo) {
   LineageU lu;
   if constexpr (Kept) {
-    const uint64_t L = r0 * A.paths + i;
-    const float4* zr = reinterpret_cast<const float4*>(A.lin_z + L * A.zrow);
-    for (uint32_t j = 0; j < steps; j += 4u) {
-      const float4 q = __ldg(zr + j / 4u);
-      zlane[j * 32u] = q.x;
-      if (j + 1u < steps) zlane[(j + 1u) * 32u] = q.y;
-      if (j + 2u < steps) zlane[(j + 2u) * 32u] = q.z;
-      if (j + 3u < steps) zlane[(j + 3u) * 32u] = q.w;
-    }
-    lu = A.lin_u[L];
+    stage_kept(A, r0, i, steps, zlane, u_age, u_one, u_one_lo);
+    return;
   } else {
     double u;
     draw_lineage(A, Z, r0, i, steps, zlane, 32u, u);
@@ -332,7 +342,7 @@ __device__ __forceinline__ void walk(const float* z, double u_age, float u1, flo
         // generation's scale ratio / paths * 2^g is applied once per row at the end
         if (w != 0.0f) kahan_add(acc + 2u * (j - 1u) * kThreads, w);
       } else {
-        const float a = Ag2[j - 1];
+        const float a = Ag2[(j - 1u) * 32u];
         if (a != 0.0f && w != 0.0f) {
           const float aw = a * w;
           f_r += aw;
@@ -413,6 +423,198 @@ __device__ __noinline__ void walk_jacobian_fp64(const float* z, double u_age, fl
   walk_jacobian(z, u_age, u1, u1_lo, inv_h, steps, stop, r, fixed_tau, acc);
 }
 
+// ---- Two walks per lane ------------------------------------------------------------------
+// The walks are bound by instruction issue, and sm_103a adds, multiplies and fuses two floats
+// per instruction. A lane takes two walks through their steps together: every FP32 operation of
+// walk() and walk_jacobian() on a pair at once, the exponential and reciprocal on each half. The
+// pair walks on while either half does; for the other half the factors are set to what leaves
+// its sums and products as they are (s = 1, 1 - s = 0 beyond kFar; a zero product once it fell
+// below the stopping level). The sums are those of the single walks bit for bit. On 256 bins,
+// 2e5 lineages and 3 types, one walk per lane -> two, with the draw tables (12 KB) gone from the
+// blocks that read kept draws: 256 candidates forward 0.958 -> 0.794, adjoint 1.109 -> 0.979,
+// Jacobian 1.186 -> 0.910 ms; 37 candidates 0.440 -> 0.344, 0.482 -> 0.395, 0.545 -> 0.356 ms; 5
+// candidates of 20,011 cells 0.100 -> 0.063, 0.108 -> 0.073 ms. A few candidates leave the
+// longest bins' blocks to themselves, and there two independent walks halve the latency; many
+// are bound by issue (1.05e9 warp instructions for the forward before). Two candidates per lane
+// instead: forward 0.859, adjoint 0.895 ms at 256, but no gain below 64.
+using f2 = float2;
+__device__ __forceinline__ f2 pair(float x) { return make_float2(x, x); }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) { return __ffma2_rn(b, pair(-1.0f), a); }  // exact product: a - b
+__device__ __forceinline__ f2 neg2(f2 a) { return make_float2(-a.x, -a.y); }
+
+// RemGrid for two walks (its operations in their order; negated constants are kept so that a
+// subtraction costs no extra negation, which rounds alike).
+struct RemGrid2 {
+  f2 C, nC, mu_g, mu_f, sg_h, nsg_h, nsg_l, t_g, t_f, Rh, Rl;
+  __device__ __forceinline__ RemGrid2(const RemGrid& a, const RemGrid& b)
+      : C(make_float2(a.C, b.C)),
+        nC(neg2(C)),
+        mu_g(make_float2(a.mu_g, b.mu_g)),
+        mu_f(make_float2(a.mu_f, b.mu_f)),
+        sg_h(make_float2(a.sg_h, b.sg_h)),
+        nsg_h(neg2(sg_h)),
+        nsg_l(make_float2(-a.sg_l, -b.sg_l)),
+        t_g(make_float2(a.t_g, b.t_g)),
+        t_f(make_float2(a.t_f, b.t_f)),
+        Rh(pair(0.0f)),
+        Rl(pair(0.0f)) {}
+  // tau = tg - ntf
+  __device__ __forceinline__ void tau(f2 z, f2& tg, f2& ntf) const {
+    const f2 ph = mul2(sg_h, z);
+    const f2 npl = fma2(nsg_l, z, fma2(nsg_h, z, ph));
+    const f2 pg = add2(add2(ph, C), nC);
+    const f2 pf = sub2(ph, pg);
+    tg = add2(mu_g, pg);
+    ntf = sub2(npl, add2(mu_f, pf));
+  }
+  __device__ __forceinline__ void first(f2 z, f2 uh, f2 ul) {
+    f2 tg, ntf;
+    tau(z, tg, ntf);
+    const f2 tf = neg2(ntf);
+    const f2 qh = mul2(tg, uh);
+    const f2 ql = fma2(tg, uh, neg2(qh));
+    const f2 rest = fma2(tf, ul, fma2(tg, ul, fma2(tf, uh, ql)));
+    const f2 qg = add2(add2(qh, C), nC);
+    const f2 qf = sub2(qh, qg);
+    Rh = sub2(t_g, qg);
+    Rl = sub2(sub2(t_f, qf), rest);
+  }
+  __device__ __forceinline__ void step(f2 z) {
+    f2 tg, ntf;
+    tau(z, tg, ntf);
+    Rh = sub2(Rh, tg);
+    Rl = add2(Rl, ntf);
+  }
+  __device__ __forceinline__ f2 x(f2 inv_h) const { return mul2(add2(Rh, Rl), inv_h); }
+};
+
+// sig_pair of both halves, with s = 1 and 1 - s = 0 for a half beyond kFar.
+__device__ __forceinline__ void sig_pair2(f2 x, f2& s, f2& one_m_s) {
+  const f2 e = make_float2(__expf(-fabsf(x.x)), __expf(-fabsf(x.y)));
+  const f2 d = add2(pair(1.0f), e);
+  const f2 q = make_float2(__fdividef(1.0f, d.x), __fdividef(1.0f, d.y));
+  const f2 eq = mul2(e, q);
+  const float q0 = x.x <= kFar ? q.x : 1.0f, q1 = x.y <= kFar ? q.y : 1.0f;
+  const float e0 = x.x <= kFar ? eq.x : 0.0f, e1 = x.y <= kFar ? eq.y : 0.0f;
+  s = make_float2(x.x >= 0.0f ? q0 : e0, x.y >= 0.0f ? q1 : e1);
+  one_m_s = make_float2(x.x >= 0.0f ? e0 : q0, x.y >= 0.0f ? e1 : q1);
+}
+
+// Two lineages of one candidate (z, 1 + U of each): walk() of the forward pass or
+// walk_jacobian(). Every generation's row takes the first lineage's term, then the second's, as
+// the single walks in turn would.
+template <bool Jacobian>
+__device__ __forceinline__ void walk_lineages(const f2* z, f2 u1, f2 u1_lo, float inv_h, uint32_t steps,
+                                              float stop, RemGrid2 r, float* acc) {
+  const f2 ih = pair(inv_h);
+  f2 zj = z[0];
+  r.first(zj, u1, u1_lo);
+  f2 dmu = mul2(u1, ih), dsig = mul2(zj, dmu);
+  f2 prod = pair(1.0f), D_mu = pair(0.0f), D_sig = pair(0.0f);
+  for (uint32_t j = 1;;) {
+    const f2 x = r.x(ih);
+    if (fminf(x.x, x.y) <= kFar) {
+      f2 s, one_m_s;
+      sig_pair2(x, s, one_m_s);
+      const f2 w = mul2(prod, one_m_s);  // leaf weights of generation j - 1
+      if constexpr (!Jacobian) {
+        float* p = acc + 2u * (j - 1u) * kThreads;
+        float sum = p[0], c = p[kThreads];
+        if (w.x != 0.0f) {  // kahan_add of each weight
+          const float y = __fsub_rn(w.x, c), t = __fadd_rn(sum, y);
+          c = __fsub_rn(__fsub_rn(t, sum), y);
+          sum = t;
+        }
+        if (w.y != 0.0f) {
+          const float y = __fsub_rn(w.y, c), t = __fadd_rn(sum, y);
+          c = __fsub_rn(__fsub_rn(t, sum), y);
+          sum = t;
+        }
+        p[kThreads] = c;
+        p[0] = sum;
+      } else {
+        float* p = acc + 3u * (j - 1u) * kThreads;
+        const f2 gm = fma2(s, dmu, D_mu), gs = fma2(s, dsig, D_sig);
+        p[0] = __fadd_rn(__fadd_rn(p[0], w.x), w.y);
+        p[kThreads] = __fmaf_rn(w.y, gm.y, __fmaf_rn(w.x, gm.x, p[kThreads]));
+        p[2 * kThreads] = __fmaf_rn(w.y, gs.y, __fmaf_rn(w.x, gs.x, p[2 * kThreads]));
+        const f2 no = neg2(one_m_s);
+        D_mu = fma2(no, dmu, D_mu);
+        D_sig = fma2(no, dsig, D_sig);
+      }
+      prod = mul2(prod, s);
+      if (fmaxf(prod.x, prod.y) < stop) break;
+      if (prod.x < stop) prod.x = 0.0f;
+      if (prod.y < stop) prod.y = 0.0f;
+    }
+    if (++j > steps) break;
+    zj = z[(j - 1) * 16u];
+    r.step(zj);
+    if constexpr (Jacobian) {
+      dmu = add2(dmu, ih);
+      dsig = fma2(zj, ih, dsig);
+    }
+  }
+}
+
+// Two lineages of one candidate for the adjoint. The per-thread sums run over a lineage's
+// generations and then over the lineages, so the second one's terms wait in shared memory
+// (`later`: weight and the two tangents per step) until the first one is through: the sums take
+// their terms in the order of the single walks.
+__device__ __forceinline__ void walk_adjoint(const f2* z, f2 u1, f2 u1_lo, float inv_h, uint32_t steps, float stop,
+                                             RemGrid2 r, float* later, const float* Ag2, float& f_r, float& f_mu,
+                                             float& f_sig) {
+  const f2 ih = pair(inv_h);
+  f2 zj = z[0];
+  r.first(zj, u1, u1_lo);
+  f2 dmu = mul2(u1, ih), dsig = mul2(zj, dmu);
+  f2 prod = pair(1.0f), D_mu = pair(0.0f), D_sig = pair(0.0f);
+  float* end = later;
+  for (uint32_t j = 1;;) {
+    const f2 x = r.x(ih);
+    if (fminf(x.x, x.y) <= kFar) {
+      f2 s, one_m_s;
+      sig_pair2(x, s, one_m_s);
+      const f2 aw = mul2(pair(Ag2[(j - 1u) * 32u]), mul2(prod, one_m_s));
+      const f2 gm = fma2(s, dmu, D_mu), gs = fma2(s, dsig, D_sig);
+      f_r = __fadd_rn(f_r, aw.x);
+      f_mu = __fmaf_rn(aw.x, gm.x, f_mu);
+      f_sig = __fmaf_rn(aw.x, gs.x, f_sig);
+      end[0] = aw.y;
+      end[kThreads] = gm.y;
+      end[2 * kThreads] = gs.y;
+      end += 3 * kThreads;
+      const f2 no = neg2(one_m_s);
+      D_mu = fma2(no, dmu, D_mu);
+      D_sig = fma2(no, dsig, D_sig);
+      prod = mul2(prod, s);
+      if (fmaxf(prod.x, prod.y) < stop) break;
+      if (prod.x < stop) prod.x = 0.0f;
+      if (prod.y < stop) prod.y = 0.0f;
+    }
+    if (++j > steps) break;
+    zj = z[(j - 1) * 16u];
+    r.step(zj);
+    dmu = add2(dmu, ih);
+    dsig = fma2(zj, ih, dsig);
+  }
+  for (const float* p = later; p != end; p += 3 * kThreads) {
+    const float aw = p[0];
+    f_r = __fadd_rn(f_r, aw);
+    f_mu = __fmaf_rn(aw, p[kThreads], f_mu);
+    f_sig = __fmaf_rn(aw, p[2 * kThreads], f_sig);
+  }
+}
+
+// The candidate in a slot of type k's order; one warp's worth of candidates is taken as it is
+// (the order only gathers candidates of similar length into a warp), which saves the launch.
+__device__ __forceinline__ uint32_t candidate_of(const SmoothArgs& A, uint32_t ncand, uint32_t k, uint32_t slot) {
+  return ncand <= 32u ? slot : A.order[(uint64_t)k * ncand + slot];
+}
+
 // Jacobian of the expected counts: block (bin, group of 32 candidates, type k). out[c][b][g][k]
 // = (sum 2^g w_g / paths, ratio_k / paths * sum 2^g dw_g/dmean, the same for sd), i.e.
 // d E_{b,g} / d(ratio_k, mean_k, sd_k); every block draws its bin's lineages itself (the
@@ -422,19 +624,20 @@ __global__ void __launch_bounds__(kThreads, Kept ? kBlocksKeptJacobian : kBlocks
                                                               uint32_t ncand, double* __restrict__ out) {
   // dynamic: per-thread sums [3 * rows][kThreads], then the lineage draws [kWarps][rows][32]
   extern __shared__ float facc[];
-  __shared__ ZigTables Z;
+  __shared__ typename std::conditional<Kept, uint32_t, ZigTables>::type Z;  // kept draws need no tables
   __shared__ double u_age[kThreads];
-  __shared__ float u_one[kThreads], u_one_lo[kThreads];
+  __shared__ __align__(8) float u_one[kThreads], u_one_lo[kThreads];
   constexpr uint32_t kWarps = kThreads / 32;
   const uint32_t b = A.bin_order[blockIdx.x], k = blockIdx.z;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t slot = blockIdx.y * 32u + lane;
   const bool live = slot < ncand;
-  const uint32_t c = live ? A.order[(uint64_t)k * ncand + slot] : 0u;
+  const uint32_t c = live ? candidate_of(A, ncand, k, slot) : 0u;
   const uint32_t KQ = A.ntypes * 3u;
   float* zbuf = facc + (size_t)3u * A.rows * kThreads + (size_t)warp * A.rows * 32u;
-  for (uint32_t i = threadIdx.x; i < sizeof(ZigTables) / 4; i += blockDim.x)
-    reinterpret_cast<uint32_t*>(&Z)[i] = __ldg(reinterpret_cast<const uint32_t*>(A.zig) + i);
+  if constexpr (!Kept)
+    for (uint32_t i = threadIdx.x; i < sizeof(ZigTables) / 4; i += blockDim.x)
+      reinterpret_cast<uint32_t*>(&Z)[i] = __ldg(reinterpret_cast<const uint32_t*>(A.zig) + i);
   for (uint32_t i = 0; i < 3u * A.rows; ++i) facc[i * kThreads + threadIdx.x] = 0.0f;
   double ratio = 0.0, mu = 0.0, sd = 0.0;
   if (live) {
@@ -451,6 +654,8 @@ __global__ void __launch_bounds__(kThreads, Kept ? kBlocksKeptJacobian : kBlocks
   RemGrid rg;
   const bool grid = opaque(grid_setup(rg, mu, sd, A.t_max, steps, 1.0 / A.inv_h));
   const RemFp64 rd{mu, sd, A.t_max, 0.0};
+  const bool pairs = opaque(grid && !quiescent && !fixed_tau);
+  const RemGrid2 rg2(rg, rg);
   const float stop = stop_level(steps);  // once per block: the walks' stopping threshold
   const uint64_t nlin = (r1 - r0) * A.paths;
   for (uint64_t base = (uint64_t)warp * 32u; base < nlin; base += 32u * kWarps) {
@@ -460,7 +665,13 @@ __global__ void __launch_bounds__(kThreads, Kept ? kBlocksKeptJacobian : kBlocks
     __syncwarp();
     const uint32_t n = (uint32_t)((nlin - base) < 32u ? (nlin - base) : 32u);
     if (live) {
-      for (uint32_t ii = 0; ii < n; ++ii) {
+      const uint32_t n2 = pairs ? n & ~1u : 0u;  // lineages taken two at a time
+      for (uint32_t ii = 0; ii < n2; ii += 2u) {
+        const uint32_t li = warp * 32u + ii;
+        walk_lineages<true>(reinterpret_cast<const f2*>(zbuf + ii), *reinterpret_cast<const f2*>(u_one + li),
+                            *reinterpret_cast<const f2*>(u_one_lo + li), inv_h, steps, stop, rg2, fmy);
+      }
+      for (uint32_t ii = n2; ii < n; ++ii) {
         const uint32_t li = warp * 32u + ii;
         if (quiescent) {
           fmy[0] += 1.0f;  // quiescent type: a leaf at generation 0 (cell.cu:69-75)
@@ -491,42 +702,44 @@ __global__ void __launch_bounds__(kThreads, Kept ? kBlocksKeptJacobian : kBlocks
 // adjoint (part[c][b][3k + q] = d(sum_g A_g E_g)/d(ratio_k, mean_k, sd_k)) of one type: block
 // (bin, group of 32 candidates, type k). Every block draws its bin's lineages itself.
 template <bool Backward, bool Kept>
-__global__ void __launch_bounds__(kThreads, Kept ? kBlocksKept : kBlocksDrawn) k_smooth(const SmoothArgs A, const double* __restrict__ params,
+__global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoint : kBlocksKept) : kBlocksDrawn) k_smooth(const SmoothArgs A, const double* __restrict__ params,
                                                      uint32_t ncand, const double* __restrict__ grad_expected,
                                                      uint32_t nvalues, const int32_t* __restrict__ vidx,
                                                      double* __restrict__ out) {
   // dynamic: compensated FP32 accumulator pairs [arows][kThreads] (forward: 2 per generation
   // row, backward: 2 per parameter), then the lineage draws z [kWarps][rows][32]
   extern __shared__ float facc[];
-  __shared__ ZigTables Z;
-  __shared__ float Ag2[Backward ? 32 : 1][kSmoothMaxRows];
+  __shared__ typename std::conditional<Kept, uint32_t, ZigTables>::type Z;  // kept draws need no tables
   __shared__ double u_age[kThreads];
-  __shared__ float u_one[kThreads], u_one_lo[kThreads];
+  __shared__ __align__(8) float u_one[kThreads], u_one_lo[kThreads];
   constexpr uint32_t kWarps = kThreads / 32;
   const uint32_t b = A.bin_order[blockIdx.x], k = blockIdx.z;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t slot = blockIdx.y * 32u + lane;
   const bool live = slot < ncand;
-  const uint32_t c = live ? A.order[(uint64_t)k * ncand + slot] : 0u;
+  const uint32_t c = live ? candidate_of(A, ncand, k, slot) : 0u;
   const uint32_t KQ = A.ntypes * 3u;
   const uint32_t arows = Backward ? 6u : 2u * A.rows;
   float* zbuf = facc + (size_t)arows * kThreads + (size_t)warp * A.rows * 32u;
-  for (uint32_t i = threadIdx.x; i < sizeof(ZigTables) / 4; i += blockDim.x)
-    reinterpret_cast<uint32_t*>(&Z)[i] = __ldg(reinterpret_cast<const uint32_t*>(A.zig) + i);
+  // adjoint: 2^g dL/dE_g [rows][32 lanes], then the waiting terms [3 rows][kThreads]
+  float* const Ag2 = facc + (size_t)(arows + A.rows) * kThreads;
+  float* const later = Ag2 + 32u * A.rows + threadIdx.x;
+  if constexpr (!Kept)
+    for (uint32_t i = threadIdx.x; i < sizeof(ZigTables) / 4; i += blockDim.x)
+      reinterpret_cast<uint32_t*>(&Z)[i] = __ldg(reinterpret_cast<const uint32_t*>(A.zig) + i);
   for (uint32_t i = 0; i < arows; ++i) facc[i * kThreads + threadIdx.x] = 0.0f;
   const uint32_t cap = __ldg(A.bin_cap + b);
   const uint32_t steps = cap + 1u;
   if constexpr (Backward) {
-    for (uint32_t i = threadIdx.x; i < 32u * kSmoothMaxRows; i += blockDim.x) {
-      const uint32_t l = i / kSmoothMaxRows, g = i % kSmoothMaxRows;
-      const uint32_t sl = blockIdx.y * 32u + l;
-      const uint32_t cc = sl < ncand ? A.order[(uint64_t)k * ncand + sl] : 0u;
+    for (uint32_t i = threadIdx.x; i < 32u * steps; i += blockDim.x) {
+      const uint32_t g = i / 32u, sl = blockIdx.y * 32u + i % 32u;
       double a = 0.0;
-      if (sl < ncand && g < A.rows && g <= cap) {
+      if (sl < ncand) {
+        const uint32_t cc = candidate_of(A, ncand, k, sl);
         const int32_t v = vidx[(uint64_t)b * A.rows + g];
         if (v >= 0) a = ldexp(grad_expected[(uint64_t)cc * nvalues + v], (int)g);
       }
-      Ag2[l][g] = (float)a;
+      Ag2[i] = (float)a;
     }
   }
   const double* my_prm = params + (uint64_t)(live ? c : 0u) * KQ + 3u * k;
@@ -540,10 +753,12 @@ __global__ void __launch_bounds__(kThreads, Kept ? kBlocksKept : kBlocksDrawn) k
   const uint64_t r0 = __ldg(A.bin_start + b), r1 = __ldg(A.bin_start + b + 1);
   float* fmy = facc + threadIdx.x;
   const float inv_h = (float)A.inv_h;
-  const float* my_ag = Backward ? Ag2[lane] : nullptr;
+  const float* my_ag = Backward ? Ag2 + lane : nullptr;
   RemGrid rg;
   const bool grid = opaque(grid_setup(rg, mu, sd, A.t_max, steps, 1.0 / A.inv_h));
   const RemFp64 rd{mu, sd, A.t_max, 0.0};
+  const bool pairs = opaque(grid && walks && !quiescent && !fixed_tau);
+  const RemGrid2 rg2(rg, rg);
   const float stop = stop_level(steps);  // once per block: the walks' stopping threshold
   // lineage i of the bin: initial cell r0 + i / paths, replica i % paths
   const uint64_t nlin = (r1 - r0) * A.paths;
@@ -556,7 +771,17 @@ __global__ void __launch_bounds__(kThreads, Kept ? kBlocksKept : kBlocksDrawn) k
     const uint32_t n = (uint32_t)((nlin - base) < 32u ? (nlin - base) : 32u);
     if (live) {
       float f_r = 0.0f, f_mu = 0.0f, f_sig = 0.0f;  // adjoint terms of these (up to) 32 lineages
-      for (uint32_t ii = 0; ii < n; ++ii) {
+      const uint32_t n2 = pairs ? n & ~1u : 0u;  // lineages taken two at a time
+      for (uint32_t ii = 0; ii < n2; ii += 2u) {
+        const uint32_t li = warp * 32u + ii;
+        const f2 u = *reinterpret_cast<const f2*>(u_one + li), u_lo = *reinterpret_cast<const f2*>(u_one_lo + li);
+        if constexpr (Backward)
+          walk_adjoint(reinterpret_cast<const f2*>(zbuf + ii), u, u_lo, inv_h, steps, stop, rg2, later, my_ag, f_r, f_mu,
+                       f_sig);
+        else
+          walk_lineages<false>(reinterpret_cast<const f2*>(zbuf + ii), u, u_lo, inv_h, steps, stop, rg2, fmy);
+      }
+      for (uint32_t ii = n2; ii < n; ++ii) {
         if (quiescent) {
           // quiescent type: a leaf at generation 0 (cell.cu:69-75)
           if constexpr (Backward) {
@@ -667,6 +892,7 @@ __global__ void __launch_bounds__(256) k_smooth_order(const double* __restrict__
 }
 
 int launch_order(const SmoothArgs& A, const double* params, uint32_t ncand, cudaStream_t st) {
+  if (ncand <= 32u) return 0;  // candidate_of
   const dim3 grid((ncand + 255u) / 256u, A.ntypes);
   k_smooth_order<<<grid, 256, 0, st>>>(params, ncand, A.ntypes, A.order);
   return (int)cudaGetLastError();
@@ -712,11 +938,15 @@ __global__ void k_smooth_jacobian_merge(const double* __restrict__ jac_raw, cons
 // r_v = log1p(E_v) - log1p(T_v) and j_v = (dE_v / dparams) / (1 + E_v),
 //   loss[c] = sum_v r_v^2, jtj[c][p][q] = sum_v j_vp j_vq, jtr[c][p] = sum_v j_vp r_v.
 // E and dE come from the Jacobian pass's raw rows as in k_smooth_jacobian_merge (same order
-// of additions). Values go through shared memory in tiles; each thread keeps the running sums
-// of up to kGnSlots outputs (upper triangle of jtj, jtr, loss) in a fixed order.
-constexpr uint32_t kGnTile = 128;
-constexpr int kGnSlots = 3;
-static_assert(kSmoothMaxTypes * 3 * (kSmoothMaxTypes * 3 + 1) / 2 + kSmoothMaxTypes * 3 + 1 <= kGnSlots * kGnTile,
+// of additions). Values go through shared memory in tiles; the outputs (upper triangle of jtj,
+// jtr, loss) are spread over the block's threads, `parts` threads per output taking every
+// parts-th value of a tile, their sums added in order at the end. The FP64 pipe (2 lanes per
+// clock per SM) bounds it: about 140 operations per value for 3 types, so log1p(target) is taken
+// once per call (k_smooth_log1p) and not once per candidate. 256 candidates, 1900 values, 3
+// types: 272 us with one thread per output and both logarithms per candidate, 153 us now.
+constexpr uint32_t kGnThreads = 256;
+constexpr int kGnSlots = 2;
+static_assert(kSmoothMaxTypes * 3 * (kSmoothMaxTypes * 3 + 1) / 2 + kSmoothMaxTypes * 3 + 1 <= kGnSlots * kGnThreads,
               "outputs per candidate exceed the block's slots");
 
 __device__ __forceinline__ void gn_pair(uint32_t o, uint32_t kq, uint32_t& a, uint32_t& b) {
@@ -737,24 +967,42 @@ __device__ __forceinline__ void gn_pair(uint32_t o, uint32_t kq, uint32_t& a, ui
   }
 }
 
-__global__ void __launch_bounds__(kGnTile) k_smooth_gauss_newton(
-    const double* __restrict__ jac_raw, const double* __restrict__ params, uint32_t per_cand, uint32_t kq,
+__global__ void __launch_bounds__(256) k_smooth_log1p(const double* __restrict__ x, uint32_t n,
+                                                     double* __restrict__ y) {
+  const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+  if (i < n) y[i] = log1p(x[i]);
+}
+
+__global__ void __launch_bounds__(kGnThreads) k_smooth_gauss_newton(
+    const double* __restrict__ jac_raw, const double* __restrict__ params, uint32_t per_cand, uint32_t kq, uint32_t tile,
     const uint32_t* __restrict__ inv_off, const uint32_t* __restrict__ inv_idx, uint32_t nvalues,
-    const double* __restrict__ target, double* __restrict__ loss, double* __restrict__ jtj,
+    const double* __restrict__ target_log, double* __restrict__ loss, double* __restrict__ jtj,
     double* __restrict__ jtr) {
-  extern __shared__ double gsm[];  // [kGnTile][kq + 1]: scaled Jacobian row, then r
-  const uint32_t c = blockIdx.x;
+  extern __shared__ double gsm[];  // [tile][kq + 1]: scaled Jacobian row, then r
+  const uint32_t c = blockIdx.x, tid = threadIdx.x;
   const uint32_t w = kq + 1u;
   const uint32_t nout = kq * (kq + 1u) / 2u + kq + 1u;
+  const uint32_t parts = nout >= kGnThreads ? 1u : kGnThreads / nout;
+  const uint32_t part = parts == 1u ? 0u : tid / nout;
   const double* src = jac_raw + (uint64_t)c * per_cand * kq;
   const double* prm = params + (uint64_t)c * kq;
+  // this thread's outputs: tid % nout of its part, or tid and tid + kGnThreads
+  uint32_t o[kGnSlots], a[kGnSlots], b[kGnSlots];
+  bool on[kGnSlots];
   double acc[kGnSlots];
 #pragma unroll
-  for (int sl = 0; sl < kGnSlots; ++sl) acc[sl] = 0.0;
-  for (uint32_t v0 = 0; v0 < nvalues; v0 += kGnTile) {
-    const uint32_t v = v0 + threadIdx.x;
-    double* row = gsm + (size_t)threadIdx.x * w;
-    if (v < nvalues) {
+  for (int sl = 0; sl < kGnSlots; ++sl) {
+    o[sl] = parts == 1u ? tid + (uint32_t)sl * kGnThreads : tid % nout;
+    on[sl] = parts == 1u ? o[sl] < nout : (sl == 0 && part < parts);
+    a[sl] = b[sl] = 0u;
+    if (on[sl]) gn_pair(o[sl], kq, a[sl], b[sl]);
+    acc[sl] = 0.0;
+  }
+  for (uint32_t v0 = 0; v0 < nvalues; v0 += tile) {
+    const uint32_t v = v0 + tid;
+    const uint32_t m = nvalues - v0 < tile ? nvalues - v0 : tile;
+    if (tid < m) {
+      double* row = gsm + (size_t)tid * w;
       double e = 0.0;
       for (uint32_t q = 0; q < kq; ++q) {
         double sum = 0.0;
@@ -764,36 +1012,32 @@ __global__ void __launch_bounds__(kGnTile) k_smooth_gauss_newton(
       }
       const double inv = 1.0 / (1.0 + e);
       for (uint32_t q = 0; q < kq; ++q) row[q] *= inv;
-      row[kq] = log1p(e) - log1p(target[v]);
-    } else {
-      for (uint32_t q = 0; q <= kq; ++q) row[q] = 0.0;
+      row[kq] = log1p(e) - target_log[v];
     }
     __syncthreads();
-    const uint32_t m = nvalues - v0 < kGnTile ? nvalues - v0 : kGnTile;
 #pragma unroll
-    for (int sl = 0; sl < kGnSlots; ++sl) {
-      const uint32_t o = threadIdx.x + (uint32_t)sl * kGnTile;
-      if (o < nout) {
-        uint32_t a, b;
-        gn_pair(o, kq, a, b);
+    for (int sl = 0; sl < kGnSlots; ++sl)
+      if (on[sl]) {
         double sum = acc[sl];
-        for (uint32_t t = 0; t < m; ++t) sum = fma(gsm[t * w + a], gsm[t * w + b], sum);
+        for (uint32_t t = part; t < m; t += parts) sum = fma(gsm[t * w + a[sl]], gsm[t * w + b[sl]], sum);
         acc[sl] = sum;
       }
-    }
     __syncthreads();
+  }
+  if (parts > 1u) {
+    if (on[0]) gsm[part * nout + o[0]] = acc[0];
+    __syncthreads();
+    if (tid < nout)
+      for (uint32_t p = 1; p < parts; ++p) acc[0] += gsm[p * nout + tid];
   }
 #pragma unroll
   for (int sl = 0; sl < kGnSlots; ++sl) {
-    const uint32_t o = threadIdx.x + (uint32_t)sl * kGnTile;
-    if (o >= nout) continue;
-    uint32_t a, b;
-    gn_pair(o, kq, a, b);
-    if (b < kq) {
-      jtj[((uint64_t)c * kq + a) * kq + b] = acc[sl];
-      jtj[((uint64_t)c * kq + b) * kq + a] = acc[sl];
-    } else if (a < kq) {
-      jtr[(uint64_t)c * kq + a] = acc[sl];
+    if (!on[sl] || part != 0u) continue;
+    if (b[sl] < kq) {
+      jtj[((uint64_t)c * kq + a[sl]) * kq + b[sl]] = acc[sl];
+      jtj[((uint64_t)c * kq + b[sl]) * kq + a[sl]] = acc[sl];
+    } else if (a[sl] < kq) {
+      jtr[(uint64_t)c * kq + a[sl]] = acc[sl];
     } else {
       loss[c] = acc[sl];
     }
@@ -811,15 +1055,15 @@ __global__ void k_smooth_grad_sum(const double* __restrict__ part, uint32_t ncan
 }
 
 // accumulator pairs (2 floats per output row and thread) + the lineage draws (kThreads
-// floats per generation row)
-int smem_bytes(uint32_t out_rows, uint32_t rows) {
-  return (int)((2u * out_rows + rows) * kThreads * sizeof(float));
+// floats per generation row) + the adjoint's gradients and waiting terms
+int smem_bytes(bool backward, uint32_t rows) {
+  return (int)((backward ? (6u + 4u * rows) * kThreads + 32u * rows : 3u * rows * kThreads) * sizeof(float));
 }
 
 template <bool Backward, bool Kept>
 int launch_smooth_k(const SmoothArgs& A, const double* params, uint32_t ncand, const double* grad_expected,
                     uint32_t nvalues, const int32_t* vidx, double* out, cudaStream_t st) {
-  const int smem = smem_bytes(Backward ? 3u : A.rows, A.rows);
+  const int smem = smem_bytes(Backward, A.rows);
   // static shared memory plus `smem` may exceed the default 48 KB: always opt in
   const cudaError_t e =
       cudaFuncSetAttribute(k_smooth<Backward, Kept>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -907,8 +1151,13 @@ int launch_smooth_gauss_newton(const SmoothArgs& A, const double* params, uint32
   }
   const int ej = launch_jacobian_k(A, params, ncand, jac_raw, st);
   if (ej != 0) return ej;
-  k_smooth_gauss_newton<<<ncand, kGnTile, kGnTile * (kq + 1u) * sizeof(double), st>>>(
-      jac_raw, params, A.nbins * A.rows, kq, inv_off, inv_idx, nvalues, target, loss, jtj, jtr);
+  double* target_log = jac_raw + (size_t)ncand * A.nbins * A.rows * kq;  // the scratch's tail
+  k_smooth_log1p<<<(nvalues + 255u) / 256u, 256, 0, st>>>(target, nvalues, target_log);
+  const uint32_t nout = kq * (kq + 1u) / 2u + kq + 1u;
+  const uint32_t tile = kq <= 18u ? 256u : 128u;  // at most 39 KB of rows
+  const size_t smem = std::max<size_t>(tile * (kq + 1u), nout < kGnThreads ? kGnThreads : 0u) * sizeof(double);
+  k_smooth_gauss_newton<<<ncand, kGnThreads, smem, st>>>(jac_raw, params, A.nbins * A.rows, kq, tile, inv_off, inv_idx,
+                                                         nvalues, target_log, loss, jtj, jtr);
   return (int)cudaGetLastError();
 }
 

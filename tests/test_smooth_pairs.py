@@ -1,0 +1,61 @@
+"""The two-walks-per-lane passes of the smoothed form where they can go wrong: bins with one,
+two, odd and just over a warp's lineages, one candidate and one more than a warp's lanes, types
+whose walks fall back to one at a time (quiescent, zero mean, the FP64 form), against the FP64
+CPU restatement with the tolerances of tests/test_smooth.py; and Gauss-Newton systems of one to
+eight types against their Jacobian."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("candidates", [1, 32, 33, 65])
+@pytest.mark.parametrize("h", [0.5, 1e-7])  # 1e-7: beyond the grid form's error bound
+def test_passes_at_their_edges(engine, candidates, h):
+    import smooth_ref
+    import torch
+    from procell.smooth import Smooth
+    bins = [(900.0, 1), (300.0, 2), (77.0, 3), (640.0, 31), (37.0, 33), (1.5, 5), (150.0, 65), (0.6, 4), (20.0, 129)]
+    sets = [[[0.5, 30.0, 6.0], [0.3, 45.0, 18.0], [0.2, -1.0, -1.0]], [[0.6, 25.0, 12.0], [0.4, 0.0, 1.0], [0.0, 40.0, 4.0]],
+            [[0.2, 60.0, 1.0], [0.5, 21.0, 9.0], [0.3, 33.0, 3.0]]]
+    rng = np.random.default_rng(3)
+    sm = Smooth(engine, bins, n_types=3, t_max=140.0, phi=1.0, h=h, paths=1, seed=99)
+    g3 = rng.normal(size=(3, sm.n_values))
+    E_ref, G_ref, vals, J_ref = smooth_ref.forward_backward(bins, 140.0, 1.0, h, 1, 99, sets, g3, with_jacobian=True)
+    pick = np.arange(candidates) % 3
+    P = torch.tensor(np.array(sets)[pick], dtype=torch.float64, device="cuda")
+    E = sm.forward(P).cpu().numpy()
+    G = sm.backward(P, torch.tensor(g3[pick], device="cuda")).cpu().numpy()
+    EJ, J = (x.cpu().numpy() for x in sm.jacobian(P))
+    sm.sync()
+    sm.close()
+    assert np.array_equal(vals, sm.values)
+    for got, ref, atol in ((E, E_ref, 1e-9), (EJ, E_ref, 1e-9), (G, G_ref, 1e-7), (J, J_ref, 1e-7)):
+        assert np.allclose(got, ref[pick], rtol=2e-5, atol=atol * np.abs(ref).max())
+        for k in range(3):  # equal candidates, equal results, wherever they stand
+            same = got[pick == k]
+            assert np.array_equal(same, np.broadcast_to(same[:1], same.shape))
+
+
+@pytest.mark.parametrize("types", [1, 2, 5, 8])
+def test_gauss_newton_of_every_width(engine, types):
+    import torch
+    from procell.smooth import Smooth
+    rng = np.random.default_rng(types)
+    bins = [(float(v), int(f)) for v, f in zip(np.exp(rng.uniform(0, 7, 41)), rng.integers(1, 9, 41))]
+    sm = Smooth(engine, bins, n_types=types, t_max=150.0, phi=1.0, h=0.5, paths=1, seed=5)
+    P = np.empty((3, types, 3))
+    P[..., 0] = rng.dirichlet(np.ones(types), 3)
+    P[..., 1] = rng.uniform(25, 70, (3, types))
+    P[..., 2] = 0.2 * P[..., 1]
+    P = torch.tensor(P, device="cuda")
+    target = torch.tensor(rng.lognormal(2.0, 1.0, sm.n_values), device="cuda")
+    loss, jtj, jtr = sm.gauss_newton(P, target)
+    E, J = sm.jacobian(P)
+    r = torch.log1p(E) - torch.log1p(target)
+    Js = (J / (1.0 + E)[:, :, None, None]).reshape(3, sm.n_values, -1)
+    # FP64 sums of at most 600 terms in another order
+    assert torch.allclose(loss, (r ** 2).sum(1), rtol=1e-12)
+    assert torch.allclose(jtj, torch.einsum("cvp,cvq->cpq", Js, Js), rtol=1e-11, atol=1e-12 * float(jtj.abs().max()))
+    assert torch.allclose(jtr, torch.einsum("cvp,cv->cp", Js, r), rtol=1e-11, atol=1e-12 * float(jtr.abs().max()))
+    sm.close()
