@@ -65,9 +65,8 @@ struct pc_context {
   // resident blocks per SM of each configuration's kernels: [narrow][batched][config]
   int occ[2][2][kNumSweepConfigs][3] = {};
   uint32_t* persist_ctl = nullptr;       // [2] barrier + [8] run totals (u64 [4])
-  // tree walk: control words, the warps' global regions (grown on demand; runs of one context
-  // follow one another), resident blocks per SM of its kernels [batched]
-  WalkCtl* walk_ctl = nullptr;
+  // tree walk: the warps' global regions (grown on demand; runs of one context follow one
+  // another), resident blocks per SM of its kernels [batched]
   void* walk_dev = nullptr;
   size_t walk_bytes = 0;
   int walk_occ[2] = {0, 0};
@@ -156,6 +155,9 @@ struct pc_plan {
   void* map_dev = nullptr;
   size_t map_bytes = 0;
   bool map_ready = false;
+  // the tables' host copy while their upload may be in flight on the context's own stream
+  std::vector<char> tables_host;
+  bool upload_pending = false;
   cudaGraphExec_t graph = nullptr;           // persistent driver: the captured run
   // ... and what it was captured with: the launch's arguments (the persistent sweeps' or the
   // tree walk's), configuration (-1: the tree walk) and grid
@@ -704,7 +706,6 @@ int pc_create(pc_context** out, int device) {
   if ((e = pc_cuda_malloc(&ctx->stats_dev, 4 * sizeof(unsigned long long))) != cudaSuccess) return bail(e, "cudaMalloc");
   if ((e = pc_cuda_malloc(&ctx->error_dev, sizeof(uint32_t))) != cudaSuccess) return bail(e, "cudaMalloc");
   if ((e = pc_cuda_malloc(&ctx->persist_ctl, 48)) != cudaSuccess) return bail(e, "cudaMalloc");
-  if ((e = pc_cuda_malloc(&ctx->walk_ctl, sizeof(WalkCtl))) != cudaSuccess) return bail(e, "cudaMalloc");
   if ((e = pc_cuda_malloc_host(&ctx->pinned, 64 * sizeof(unsigned long long))) != cudaSuccess)
     return bail(e, "cudaMallocHost");
   for (auto& ev : ctx->ev)
@@ -723,7 +724,11 @@ void pc_destroy(pc_context* ctx) {
   if (ctx->stream) pc_cuda_sync(ctx->stream);
   if (ctx->copy_stream) pc_cuda_sync(ctx->copy_stream);
   free_pool(ctx);
-  for (pc_plan* p : ctx->live) p->owner = nullptr;  // plans outliving their context free their own buffers
+  for (pc_plan* p : ctx->live) {
+    p->owner = nullptr;  // plans outliving their context free their own buffers
+    if (p->upload_pending) cudaStreamSynchronize(ctx->own_stream);
+    p->upload_pending = false;
+  }
   for (int i = 0; i < kSpares; ++i) {
     pc_cuda_free(ctx->spare_rec[i].p);
     pc_cuda_free(ctx->spare_hist[i].p);
@@ -736,7 +741,6 @@ void pc_destroy(pc_context* ctx) {
   pc_cuda_free(ctx->stats_dev);
   pc_cuda_free(ctx->error_dev);
   pc_cuda_free(ctx->persist_ctl);
-  pc_cuda_free(ctx->walk_ctl);
   pc_cuda_free(ctx->walk_dev);
   cudaFreeHost(ctx->pinned);
   cudaFreeHost(ctx->stage);
@@ -1115,6 +1119,19 @@ int finalize_host(pc_plan* p, uint64_t max_root_chunk, PlanTables& t, std::strin
   return PC_OK;
 }
 
+// A plan's table upload is known to be done: its host copy goes.
+void upload_done(pc_plan* p) {
+  p->upload_pending = false;
+  std::vector<char>().swap(p->tables_host);
+}
+// Waits for a plan's table upload, in flight on the context's own stream (or on `st`).
+cudaError_t wait_upload(pc_context* ctx, pc_plan* p, cudaStream_t st = nullptr) {
+  if (!p->upload_pending) return cudaSuccess;
+  const cudaError_t e = pc_cuda_sync(st ? st : ctx->own_stream);
+  if (e == cudaSuccess) upload_done(p);
+  return e;
+}
+
 // The allocations and uploads of a plan whose host part is done (on the context's thread).
 int finalize_device(pc_context* ctx, pc_plan* p, const PlanTables& t) {
   const auto& bin_inst = t.bin_inst;
@@ -1157,28 +1174,32 @@ int finalize_device(pc_context* ctx, pc_plan* p, const PlanTables& t) {
     }
   }
   if (e == cudaSuccess)
-    e = take_spare(ctx->spare_hist, p->hist_elems * sizeof(unsigned long long),
+    e = take_spare(ctx->spare_hist, p->hist_elems * sizeof(unsigned long long) + sizeof(WalkCtl),
                    reinterpret_cast<void**>(&p->hist_dev), &p->hist_bytes);
-  if (e == cudaSuccess && nb)
-    e = pc_cuda_copy(p->bin_info_dev, p->bin_info.data(), nb * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess)
-    e = pc_cuda_copy(p->bin_start_dev, p->bin_start.data(), (nb + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st);
+  // one copy of all tables, from memory that the plan keeps until the copy is known to be done
+  // (the first run's synchronisation, or pc_plan_destroy); on a caller's stream, which may be
+  // gone by then, it is waited for here
+  p->tables_host.resize(tables);
+  auto put = [p](size_t at, const void* src, size_t bytes) {
+    if (bytes) std::memcpy(p->tables_host.data() + at, src, bytes);
+  };
+  put(o_info, p->bin_info.data(), nb * sizeof(uint32_t));
+  put(o_start, p->bin_start.data(), (nb + 1) * sizeof(uint64_t));
   if (!p->batched) {
-    if (e == cudaSuccess)
-      e = pc_cuda_copy(p->types_dev, p->inst[0].types.data(), nt * sizeof(TypeDev), cudaMemcpyHostToDevice, st);
+    put(o_types, p->inst[0].types.data(), nt * sizeof(TypeDev));
     p->upload_bytes += nt * sizeof(TypeDev);
   } else {
-    if (e == cudaSuccess)
-      e = pc_cuda_copy(p->btypes_dev, btypes.data(), btypes.size() * sizeof(BatchType), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-      e = pc_cuda_copy(p->inst_dev, idev.data(), idev.size() * sizeof(InstanceDev), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && nb)
-      e = pc_cuda_copy(p->bin_inst_dev, bin_inst.data(), nb * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && nb)
-      e = pc_cuda_copy(p->bin_class_dev, bin_class.data(), nb * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
+    put(o_btypes, btypes.data(), btypes.size() * sizeof(BatchType));
+    put(o_inst, idev.data(), idev.size() * sizeof(InstanceDev));
+    put(o_binst, bin_inst.data(), nb * sizeof(uint32_t));
+    put(o_bclass, bin_class.data(), nb * sizeof(uint32_t));
     p->upload_bytes += btypes.size() * sizeof(BatchType) + idev.size() * sizeof(InstanceDev) + 2 * nb * sizeof(uint32_t);
   }
-  if (e == cudaSuccess) e = pc_cuda_sync(st);
+  if (e == cudaSuccess) {
+    p->upload_pending = true;
+    e = pc_cuda_copy(p->tables_dev, p->tables_host.data(), tables, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && st != ctx->own_stream) e = wait_upload(ctx, p, st);
+  }
   if (e != cudaSuccess)
     return fail(ctx, e == cudaErrorMemoryAllocation ? PC_ERR_NOMEM : PC_ERR_CUDA,
                 std::string("plan upload: ") + cudaGetErrorString(e));
@@ -1609,6 +1630,7 @@ int pc_plan_set_roots(pc_context* ctx, pc_plan* p, uint64_t root_begin, uint64_t
 void pc_plan_destroy(pc_plan* p) {
   if (!p) return;
   if (p->graph) cudaGraphExecDestroy(p->graph);
+  if (p->upload_pending && p->owner) cudaStreamSynchronize(p->owner->own_stream);
   if (p->owner) {
     pc_context* ctx = p->owner;
     ctx->live.erase(std::remove(ctx->live.begin(), ctx->live.end(), p), ctx->live.end());
@@ -1940,10 +1962,10 @@ bool walk_serves(const pc_context* ctx, const pc_plan* p) {
 
 // The operations of one tree walk, in stream order (also what a graph captures).
 int enqueue_walk(pc_context* ctx, pc_plan* p, const WalkArgs& w, int grid, cudaStream_t s) {
-  PC_CUDA(ctx, pc_cuda_memset(p->hist_dev, 0, p->hist_elems * sizeof(unsigned long long), s));
-  PC_CUDA(ctx, pc_cuda_memset(ctx->walk_ctl, 0, sizeof(WalkCtl), s));
+  // the control words lie behind the counts: one clear for both
+  PC_CUDA(ctx, pc_cuda_memset(p->hist_dev, 0, p->hist_elems * sizeof(unsigned long long) + sizeof(WalkCtl), s));
   PC_CUDA(ctx, PC_LAUNCH(launch_walk(w, grid, s)));
-  PC_CUDA(ctx, pc_cuda_copy(ctx->pinned + 24, ctx->walk_ctl, offsetof(WalkCtl, barrier), cudaMemcpyDeviceToHost, s));
+  PC_CUDA(ctx, pc_cuda_copy(ctx->pinned + 24, w.ctl, offsetof(WalkCtl, barrier), cudaMemcpyDeviceToHost, s));
   return PC_OK;
 }
 
@@ -1968,8 +1990,8 @@ int run_walk(pc_context* ctx, pc_plan* p, const RunArgs& a) {
   w.a.root_rec = nullptr;
   w.a.rec_cap = 0;
   w.a.stats = nullptr;
-  w.a.error = &ctx->walk_ctl->error;
-  w.ctl = ctx->walk_ctl;
+  w.ctl = reinterpret_cast<WalkCtl*>(p->hist_dev + p->hist_elems);
+  w.a.error = &w.ctl->error;
   w.root_lo = p->root_begin;
   w.root_hi = p->root_end;
   w.batch = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(4, (nroots + warps - 1) / warps));
@@ -2107,6 +2129,7 @@ int pc_plan_run(pc_context* ctx, pc_plan* p) {
   // a run that failed part way may have left level buffers marked in use; every run is
   // complete (or failed) when its call returns, and work in flight is ordered on the stream
   for (auto& lb : ctx->pool) lb.busy = false;
+  if (st != ctx->own_stream) PC_CUDA(ctx, wait_upload(ctx, p));
   std::memset(&p->stats, 0, sizeof(p->stats));
   const uint64_t nroots = p->root_end - p->root_begin;
   p->stats.roots = nroots;
@@ -2143,6 +2166,7 @@ int pc_plan_run(pc_context* ctx, pc_plan* p) {
     rc = run_per_sweep(ctx, p, K, occ, a);
   }
   if (rc != PC_OK) return rc;
+  if (p->upload_pending) upload_done(p);  // the run ended with a synchronisation of its stream
   p->stats.vanished = ctx->pinned[0];
   p->stats.uncounted = ctx->pinned[1];
   p->stats.h2d_bytes = p->upload_bytes;
@@ -2389,6 +2413,7 @@ int pc_batch_set_types(pc_context* ctx, pc_batch* b, const pc_cell_type* types) 
   batch_type_tables(b, btypes, idev);
   b->ran = false;  // counts of the previous run belong to the previous types
   PC_CUDA(ctx, cudaSetDevice(ctx->device));
+  PC_CUDA(ctx, wait_upload(ctx, b));
   PC_CUDA(ctx, pc_cuda_copy(b->btypes_dev, btypes.data(), btypes.size() * sizeof(BatchType),
                                cudaMemcpyHostToDevice, ctx->stream));
   PC_CUDA(ctx, pc_cuda_copy(b->inst_dev, idev.data(), idev.size() * sizeof(InstanceDev), cudaMemcpyHostToDevice,
