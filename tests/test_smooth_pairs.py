@@ -37,6 +37,43 @@ def test_passes_at_their_edges(engine, candidates, h):
             assert np.array_equal(same, np.broadcast_to(same[:1], same.shape))
 
 
+@pytest.mark.parametrize("depth", [1, 33, 63])  # 63: the most generations a bin may have
+@pytest.mark.parametrize("lineages", [2, 35])
+def test_pairs_against_single_walks(engine, depth, lineages):
+    """The same lineages in one bin (walked in pairs) and in one bin each (walked alone; values a
+    little apart, so that every lineage's results can be told). A weight has the same factors
+    either way, so the sums differ by their roundings, 2^-24 of the sum of magnitudes per term, and
+    by what pairs add below the stopping level, e^-40 cells (times a tangent below 1e5). Types that
+    divide to the end, that stop on the way, and with factors below the normal floats."""
+    import torch
+    from procell.smooth import Smooth
+    v = 1.5 * 2.0 ** depth
+    apart = [v * (1.0 + i / 1024.0) for i in range(lineages)]
+    P = torch.tensor([[[0.5, 2.1, 0.2], [0.3, 9.0, 3.0], [0.2, 300.0, 10.0]]], dtype=torch.float64, device="cuda")
+    rng = np.random.default_rng(depth)
+    gen_grad = rng.normal(size=depth + 1) * 0.5 ** np.arange(depth + 1)
+    E, J, G = [], [], []
+    for bins in ([(v, lineages)], [(a, 1) for a in apart]):
+        sm = Smooth(engine, bins, n_types=3, t_max=140.0, phi=1.0, h=0.5, paths=1, seed=17)
+        values = list(sm.values)
+        idx = np.array([[values.index(x / 2.0 ** g) for g in range(depth + 1)] for x, _ in bins])
+        grad = np.zeros((1, sm.n_values))
+        grad[0, idx] = gen_grad
+        e, j = (x.cpu().numpy() for x in sm.jacobian(P))
+        E.append((sm.forward(P).cpu().numpy()[0, idx], e[0, idx]))
+        J.append(j[0, idx])
+        G.append(sm.backward(P, torch.tensor(grad, device="cuda")).cpu().numpy()[0])
+        sm.sync()
+        sm.close()
+    eps = (lineages + 2) * 2.0 ** -24
+    for pair, single in zip(*E):
+        assert np.all(np.abs(pair[0] - single.sum(0)) <= eps * single.sum(0) + 1e-15)
+    mags = np.abs(J[1]).sum(0)
+    assert np.all(np.abs(J[0][0] - J[1].sum(0)) <= eps * mags + 1e-10)
+    terms = np.einsum("g,gkq->kq", np.abs(gen_grad), mags)
+    assert np.all(np.abs(G[0] - G[1]) <= (64 * lineages + 2) * 2.0 ** -24 * terms + 1e-10)
+
+
 @pytest.mark.parametrize("types", [1, 2, 5, 8])
 def test_gauss_newton_of_every_width(engine, types):
     import torch
