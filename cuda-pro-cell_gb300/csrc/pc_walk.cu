@@ -3,11 +3,13 @@
 
 namespace pc {
 
+static size_t walk_smem_bytes(bool batched) { return batched ? sizeof(WalkSmem<true>) : sizeof(WalkSmem<false>); }
+
 int walk_occupancy(bool batched, int* blocks_per_sm) {
   auto* k = batched ? k_walk<true> : k_walk<false>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkSmem));
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, kWalkThreads, sizeof(WalkSmem));
+  const size_t smem = walk_smem_bytes(batched);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, kWalkThreads, smem);
   return (int)e;
 }
 
@@ -17,7 +19,7 @@ int launch_walk(const WalkArgs& w, int blocks, void* stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3((unsigned)kWalkThreads);
-  cfg.dynamicSmemBytes = sizeof(WalkSmem);
+  cfg.dynamicSmemBytes = walk_smem_bytes(w.a.btypes != nullptr);
   cfg.stream = (cudaStream_t)stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;

@@ -14,7 +14,7 @@
 //   the exact FP64 due time the level sweeps compare. A daughter with |rem| <= band (about 1
 //   in 20000), like one whose first-attempt normal is rejected or not certainly inside the
 //   truncation tau > 0, is parked and settled 32 at a time: its normal by the generic
-//   sampler and, inside the band, its due time by replaying its lineage from the initial
+//   sampler and, still inside the band, its due time by replaying its lineage from the initial
 //   cell in FP64 with the operations of the sweeps. Counts are therefore bit-identical, and
 //   the FP64 pipe does nothing for the other 99.99%.
 //
@@ -35,7 +35,7 @@
 // (23 cycles alone) and 33 shared-memory wavefronts, half of those the ziggurat's random lookups;
 // measured alone it takes 50 cycles of an SM, 5.0 ps per division, and adding warps (24 to 32 per
 // SM) changes that by 4%. A whole run of 2.27e9 divisions takes 13.1 ms, 5.8 ps per division,
-// against 10.1 ps for the level sweeps; a run of 14e6 divisions of 1e6 initial cells 0.20 ms
+// against 10.1 ps for the level sweeps; a run of 14e6 divisions of 1e6 initial cells 0.19 ms
 // against 0.45 ms; 16 thousand divisions 0.033 ms against 0.16 ms and nine host round trips.
 // 24 warps per SM with stacks of 400 cells, because a spill of 32 cells and their return cost
 // about 350 instructions: 32 warps and 264 cells 14.0 ms, 28 and 320 13.2, 24 and 400 13.1, 20
@@ -53,9 +53,16 @@ constexpr int kWalkThreads = 768;
 constexpr int kWalkWarps = kWalkThreads / 32;
 constexpr int kWalkBlocksPerSm = 1;
 constexpr uint32_t kCols = kWalkCols;   // histogram classes in a warp's window
-constexpr uint32_t kStackCap = 400;     // shared-memory stack entries of a warp, parked ones included
-constexpr uint32_t kStackRoom = kStackCap - 96u - 31u;  // cells a full step may start with: it pops 32 and
-                                                        // adds at most 128, with up to 31 parked before it
+// Shared-memory stack entries of a warp, parked ones included, and the cells a full step may start
+// with: it pops 32 and adds at most 128, with up to 31 parked before it. A batched run refills its
+// stacks far more often than it overflows them, and its lookups and the local memory of the code
+// around the steps gain more from 32 KB more of L1 than its steps from 80 more cells: 25.6e6
+// initial cells and 1.29e8 divisions 1.86 ms with 400, 1.68 with 320, a plain run of 2.27e9
+// divisions 13.05 and 13.27 ms.
+template <bool Batched>
+constexpr uint32_t kStackCap = Batched ? 320 : 400;
+template <bool Batched>
+constexpr uint32_t kStackRoom = kStackCap<Batched> - 96u - 31u;
 constexpr uint32_t kFirstPoll = 8;      // steps of a round before the first look at the idle warps
 constexpr uint32_t kPollSteps = 32;     // steps between two looks at the number of idle warps
 constexpr uint32_t kIdlePolls = 120;    // looks that found any idle warp after which cells are handed over
@@ -80,6 +87,7 @@ constexpr uint32_t kMetaDeeper = 30u << kMetaLeftShift;  // nonzero: its daughte
 constexpr uint32_t kMetaChild = 4u + (1u << kMetaLeftShift);
 static_assert(kWalkMaxGen < kColWords && kCols <= 16, "one word per generation to go; four bits of column");
 
+template <bool Batched>
 struct alignas(16) WalkWarp {
   float4 rec[kCols];  // mean, sd, eps, band of the column's type
   uint2 key[kCols];   // its instance's seed
@@ -87,8 +95,8 @@ struct alignas(16) WalkWarp {
   uint32_t window[kCols * kColWords];
   // the stack: cells from the bottom, parked daughters from the top; two arrays, so that a
   // step's two daughters share the registers of their second half
-  uint2 stack_t[kStackCap];  // time left, node
-  uint2 stack_m[kStackCap];  // initial cell, meta
+  uint2 stack_t[kStackCap<Batched>];  // time left, node
+  uint2 stack_m[kStackCap<Batched>];  // initial cell, meta
   // the round's state, out of the step's registers (uniform over the warp, written by lane 0)
   unsigned long long cpos, cend;                      // current range of initial cells
   unsigned long long divisions, vanished, uncounted;  // totals of the round so far
@@ -97,9 +105,10 @@ struct alignas(16) WalkWarp {
   uint32_t taken, pad;  // supplies taken (0: none yet)
 };
 
+template <bool Batched>
 struct alignas(16) WalkSmem {
   uint2 zig[kZigLayers];  // strip-test bound and scale of each ziggurat layer
-  WalkWarp warp[kWalkWarps];
+  WalkWarp<Batched> warp[kWalkWarps];
   uint32_t finished;  // warps of the block that have finished the round
   uint32_t pad[3];
   WalkArgs w;  // the launch's arguments, for the code outside the step
@@ -114,8 +123,14 @@ __device__ __forceinline__ T* shared_at(uint32_t address) {
 }
 
 extern __shared__ __align__(16) unsigned char walk_smem[];
-__device__ __forceinline__ WalkSmem& walk_shared() { return *reinterpret_cast<WalkSmem*>(walk_smem); }
-__device__ __forceinline__ WalkWarp& walk_warp() { return walk_shared().warp[threadIdx.x >> 5]; }
+template <bool Batched>
+__device__ __forceinline__ WalkSmem<Batched>& walk_shared() {
+  return *reinterpret_cast<WalkSmem<Batched>*>(walk_smem);
+}
+template <bool Batched>
+__device__ __forceinline__ WalkWarp<Batched>& walk_warp() {
+  return walk_shared<Batched>().warp[threadIdx.x >> 5];
+}
 
 // The exact due time of a node, by its lineage from the initial cell: the operations of
 // root_body and divide_body (pc_sweeps.cuh), in their order.
@@ -145,14 +160,19 @@ __device__ __forceinline__ const TypeDev& walk_type(const RunArgs& a, uint32_t t
 }
 
 // Checked build: a stack index in range (true at compile time otherwise).
-__device__ __forceinline__ bool stack_ok(uint32_t i) { return in_bounds(i < kStackCap, walk_shared().w.a.error); }
-__device__ __forceinline__ uint4 stack_get(const WalkWarp& W, uint32_t i) {
-  if (!stack_ok(i)) return make_uint4(0u, 0u, 0u, 0u);
+template <bool Batched>
+__device__ __forceinline__ bool stack_ok(uint32_t i) {
+  return in_bounds(i < kStackCap<Batched>, walk_shared<Batched>().w.a.error);
+}
+template <bool Batched>
+__device__ __forceinline__ uint4 stack_get(const WalkWarp<Batched>& W, uint32_t i) {
+  if (!stack_ok<Batched>(i)) return make_uint4(0u, 0u, 0u, 0u);
   const uint2 t = W.stack_t[i], m = W.stack_m[i];
   return make_uint4(t.x, t.y, m.x, m.y);
 }
-__device__ __forceinline__ void stack_put(WalkWarp& W, uint32_t i, uint4 e) {
-  if (!stack_ok(i)) return;
+template <bool Batched>
+__device__ __forceinline__ void stack_put(WalkWarp<Batched>& W, uint32_t i, uint4 e) {
+  if (!stack_ok<Batched>(i)) return;
   W.stack_t[i] = make_uint2(e.x, e.y);
   W.stack_m[i] = make_uint2(e.z, e.w);
 }
@@ -170,9 +190,10 @@ __device__ __forceinline__ uint4* walk_region(const WalkArgs& w, uint32_t round)
 
 // The window into the global table: leaves(g) = 2 D(g - 1) - D(g) - (g == cap ? V : 0), in
 // wrapping arithmetic (a cell handed over is counted by another warp than its parent).
+template <bool Batched>
 __device__ __noinline__ void walk_flush(uint32_t ncols) {
-  const RunArgs& a = walk_shared().w.a;
-  WalkWarp& W = walk_warp();
+  const RunArgs& a = walk_shared<Batched>().w.a;
+  WalkWarp<Batched>& W = walk_warp<Batched>();
   const uint32_t lane = threadIdx.x & 31u;
   unsigned long long divisions = 0, vanished = 0;
   uint32_t gens = 0;  // bit g: a cell of generation g divided
@@ -206,7 +227,8 @@ __device__ __noinline__ void walk_flush(uint32_t ncols) {
 }
 
 // The 32 bottom cells of a full stack of `n` cells to the warp's global region.
-__device__ __forceinline__ void walk_spill(const WalkArgs& w, WalkWarp& W, uint32_t round, uint32_t n) {
+template <bool Batched>
+__device__ __forceinline__ void walk_spill(const WalkArgs& w, WalkWarp<Batched>& W, uint32_t round, uint32_t n) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t nspill = W.nspill;
   uint4 low = stack_get(W, lane);
@@ -230,7 +252,7 @@ __device__ __forceinline__ void walk_spill(const WalkArgs& w, WalkWarp& W, uint3
 // One step: up to 32 dividing cells off the stack (Full: exactly 32), both daughters of each.
 // Returns whether daughters were parked.
 template <bool Batched, bool Full>
-__device__ __forceinline__ bool walk_step(const uint32_t* ks, const WalkSmem& S, WalkWarp& W, uint32_t lane,
+__device__ __forceinline__ bool walk_step(const uint32_t* ks, const WalkSmem<Batched>& S, WalkWarp<Batched>& W, uint32_t lane,
                                           uint32_t lt, uint32_t& sp, uint32_t& np) {
   const uint32_t n = Full ? 32u : min(sp, 32u);
   const uint32_t base = sp - n;
@@ -270,14 +292,14 @@ __device__ __forceinline__ bool walk_step(const uint32_t* ks, const WalkSmem& S,
   const uint2 child = make_uint2(root, meta - kMetaChild);
   if (go0) {
     const uint32_t at = base + __popc(b0 & lt);
-    if (stack_ok(at)) {
+    if (stack_ok<Batched>(at)) {
       W.stack_t[at] = make_uint2(__float_as_uint(r0), 2u * node);
       W.stack_m[at] = child;
     }
   }
   if (go1) {
     const uint32_t at = base + c0 + __popc(b1 & lt);
-    if (stack_ok(at)) {
+    if (stack_ok<Batched>(at)) {
       W.stack_t[at] = make_uint2(__float_as_uint(r1), 2u * node + 1u);
       W.stack_m[at] = child;
     }
@@ -287,7 +309,7 @@ __device__ __forceinline__ bool walk_step(const uint32_t* ks, const WalkSmem& S,
   const bool parked = __any_sync(kFull, p0 | p1);
   if (parked) {
     const uint32_t k0 = __ballot_sync(kFull, p0), k1 = __ballot_sync(kFull, p1);
-    const uint32_t at = kStackCap - 1u - np - __popc(k0 & lt) - __popc(k1 & lt);
+    const uint32_t at = kStackCap<Batched> - 1u - np - __popc(k0 & lt) - __popc(k1 & lt);
     if (p0) stack_put(W, at, make_uint4(et.x, 2u * node, child.x, child.y));
     if (p1) stack_put(W, at - (p0 ? 1u : 0u), make_uint4(et.x, 2u * node + 1u, child.x, child.y));
     np += __popc(k0) + __popc(k1);
@@ -300,7 +322,8 @@ __device__ __forceinline__ bool walk_step(const uint32_t* ks, const WalkSmem& S,
 // wedge or a truncated timer (the first two words of the node's stream) settle all but about
 // 1% of them, with every lane on the same instructions; the rest (tails, second rejections)
 // go through the sampler's loop (slow_z), which gives the same value from the start.
-__device__ __forceinline__ float parked_z(const WalkSmem& S, const RunArgs& a, uint32_t node, uint32_t root, uint2 key,
+template <bool Batched>
+__device__ __forceinline__ float parked_z(const WalkSmem<Batched>& S, const RunArgs& a, uint32_t node, uint32_t root, uint2 key,
                                           float zlo, float zhi) {
   const uint32_t c = node & 1u;
   const u32x4 P = philox(u32x4{node >> 1, 0u, root, kPurposePair}, key.x, key.y);
@@ -327,27 +350,33 @@ __device__ __forceinline__ float parked_z(const WalkSmem& S, const RunArgs& a, u
 
 // Settles up to 32 parked daughters; those that divide again go on the stack.
 template <bool Batched>
-__device__ __forceinline__ void walk_settle(const WalkSmem& S, WalkWarp& W, uint32_t lane, uint32_t lt, uint32_t& sp,
-                                            uint32_t& np) {
+__device__ __forceinline__ void walk_settle(const WalkSmem<Batched>& S, WalkWarp<Batched>& W, uint32_t lane,
+                                            uint32_t lt, uint32_t& sp, uint32_t& np) {
   const RunArgs& a = S.w.a;
   const uint32_t n = min(np, 32u);
   bool emit = false;
   uint32_t vanished = 0, uncounted = 0;
   uint4 e = make_uint4(0u, 0u, 0u, 0u);
   if (lane < n) {
-    e = stack_get(W, kStackCap - np + lane);
+    e = stack_get(W, kStackCap<Batched> - np + lane);
     const uint32_t col = e.w >> kMetaColShift;
     const uint2 x = W.aux[col], key = W.key[col];
     const float4 t = W.rec[col];
     const TypeDev& T = walk_type<Batched>(a, x.y & 0xFFFFu);
     const float zlo = __ldg(&T.zlo), zhi = __ldg(&T.zhi);
     const bool initial = e.y == 1u;
-    float rem = 0.0f;
-    if (!initial)
-      rem = __fsub_rn(__uint_as_float(e.x), __fmaf_rn(t.y, parked_z(S, a, e.y, e.z, key, zlo, zhi), t.x));
+    const double t_max = __ldg(&T.t_max);
+    float left = __uint_as_float(e.x), tau = __fmaf_rn(t.y, parked_z(S, a, e.y, e.z, key, zlo, zhi), t.x);
+    // An initial cell's e.x is 1 + U, and its time left is found as in walk_roots: replaying all of
+    // them in FP64 (one in most batches of 32) cost more than the rest of the settling, 0.12 ms
+    // of 2.03 for 25.6e6 initial cells against 0.04 of 1.86.
+    if (initial) {
+      tau = __fmul_rn(tau, left);
+      left = (float)t_max;
+    }
+    float rem = __fsub_rn(left, tau);
     bool leaf = rem < 0.0f;
-    if (initial || !(fabsf(rem) > t.w)) {
-      const double t_max = __ldg(&T.t_max);
+    if (!(fabsf(rem) > t.w)) {
       const double due =
           replay_due(e.y, e.z, __ldg(&T.mu), __ldg(&T.sigma), zlo, zhi, key.x, key.y, *a.zig, a.error);
       leaf = gt_nonneg(due, t_max);
@@ -383,8 +412,8 @@ __device__ __forceinline__ void walk_settle(const WalkSmem& S, WalkWarp& W, uint
 // The next up to `batch` initial cells of the warp's range: type, first timer, initial age;
 // those that divide go on the stack, unsettled ones to the parked daughters.
 template <bool Batched>
-__device__ __forceinline__ void walk_roots(const WalkSmem& S, WalkWarp& W, uint32_t lane, uint32_t lt, uint32_t& sp,
-                                           uint32_t& np) {
+__device__ __forceinline__ void walk_roots(const WalkSmem<Batched>& S, WalkWarp<Batched>& W, uint32_t lane,
+                                           uint32_t lt, uint32_t& sp, uint32_t& np) {
   const RunArgs& a = S.w.a;
   const uint64_t cpos = W.cpos, cend = W.cend;
   // bin of the first one: the one before continues, or by 32-way search the largest b with
@@ -498,7 +527,7 @@ __device__ __forceinline__ void walk_roots(const WalkSmem& S, WalkWarp& W, uint3
                                  (col << kMetaColShift));
   const uint32_t em = __ballot_sync(kFull, emit), pk = __ballot_sync(kFull, park);
   if (emit) stack_put(W, sp + __popc(em & lt), e);
-  if (park) stack_put(W, kStackCap - 1u - np - __popc(pk & lt), e);
+  if (park) stack_put(W, kStackCap<Batched> - 1u - np - __popc(pk & lt), make_uint4(__float_as_uint(one_u), e.y, e.z, e.w));
   sp += __popc(em);
   np += __popc(pk);
   const uint32_t took = min(want, limit);
@@ -516,9 +545,10 @@ __device__ __forceinline__ void walk_roots(const WalkSmem& S, WalkWarp& W, uint3
 
 // Hands the warp's cells over to the next round: the stack after the spilled ones, the columns'
 // types, and the initial cells it has taken but not begun.
+template <bool Batched>
 __device__ __noinline__ void walk_hand_over(uint32_t round, uint32_t sp) {
-  const WalkArgs& w = walk_shared().w;
-  WalkWarp& W = walk_warp();
+  const WalkArgs& w = walk_shared<Batched>().w;
+  WalkWarp<Batched>& W = walk_warp<Batched>();
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t wid = blockIdx.x * kWalkWarps + (threadIdx.x >> 5);
   const uint32_t nspill = W.nspill, ncols = W.ncols;
@@ -550,14 +580,15 @@ __device__ __noinline__ void walk_hand_over(uint32_t round, uint32_t sp) {
       w.ranges[round & 1u][k] = make_ulonglong2(W.cpos, W.cend);
     }
   }
-  walk_flush(ncols);
+  walk_flush<Batched>(ncols);
 }
 
 // The warp's next supply: a range of initial cells (round 0, or part of one given back), or a
 // range of the cells handed over, which it then loads from one source after another.
+template <bool Batched>
 __device__ __noinline__ void walk_supply(uint32_t round) {
-  const WalkArgs& w = walk_shared().w;
-  WalkWarp& W = walk_warp();
+  const WalkArgs& w = walk_shared<Batched>().w;
+  WalkWarp<Batched>& W = walk_warp<Batched>();
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t nwarps = gridDim.x * kWalkWarps;
   WalkRound& R = w.ctl->round[round & 3u];
@@ -610,9 +641,10 @@ __device__ __noinline__ void walk_supply(uint32_t round) {
 // The next cells of the warp's range of cells handed over, those of one source, with the
 // source's columns after the window's own. Returns the cells put on the stack (0: the window
 // has no room for the columns).
+template <bool Batched>
 __device__ __noinline__ uint32_t walk_load(uint32_t round, uint32_t sp) {
-  const WalkArgs& w = walk_shared().w;
-  WalkWarp& W = walk_warp();
+  const WalkArgs& w = walk_shared<Batched>().w;
+  WalkWarp<Batched>& W = walk_warp<Batched>();
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t old = (round - 1u) & 1u;
   const uint32_t lpos = W.lpos, lend = W.lend, ncols = W.ncols;
@@ -661,8 +693,8 @@ constexpr uint32_t kWalkDone = ~0u;
 
 template <bool Batched>
 __device__ __noinline__ uint32_t walk_manage(const uint32_t round, uint32_t sp, uint32_t np, const uint32_t steps) {
-  const WalkSmem& S = walk_shared();
-  WalkWarp& W = walk_warp();
+  const WalkSmem<Batched>& S = walk_shared<Batched>();
+  WalkWarp<Batched>& W = walk_warp<Batched>();
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt = (1u << lane) - 1u;
   uint32_t recent = W.recent + steps;  // steps since the last look at the idle warps
@@ -685,7 +717,7 @@ __device__ __noinline__ uint32_t walk_manage(const uint32_t round, uint32_t sp, 
       hand_over = W.lpos >= W.lend && (polls >= kIdlePolls || (polls >= kIdlePolls / kShortPolls &&
                                                                sp + W.nspill >= kLongStack));
       const bool full = walked >= (1u << 25);  // long before a 32-bit counter of the window wraps
-      if (full) walk_flush(W.ncols);
+      if (full) walk_flush<Batched>(W.ncols);
       __syncwarp();
       if (lane == 0u) {
         W.polls = polls;
@@ -694,10 +726,10 @@ __device__ __noinline__ uint32_t walk_manage(const uint32_t round, uint32_t sp, 
       continue;
     }
     if (hand_over) {
-      walk_hand_over(round, sp);
+      walk_hand_over<Batched>(round, sp);
       return kWalkDone;
     }
-    if (sp > kStackRoom) {
+    if (sp > kStackRoom<Batched>) {
       walk_spill(S.w, W, round, sp);
       sp -= 32u;
       continue;
@@ -720,13 +752,13 @@ __device__ __noinline__ uint32_t walk_manage(const uint32_t round, uint32_t sp, 
       if (W.cpos < W.cend)
         walk_roots<Batched>(S, W, lane, lt, sp, np);
       else if (W.lpos < W.lend)
-        sp += walk_load(round, sp);
+        sp += walk_load<Batched>(round, sp);
       else
-        walk_supply(round);
+        walk_supply<Batched>(round);
       continue;
     }
     if (sp == 0u) {  // nothing left here (np == 0: settled above)
-      walk_flush(W.ncols);
+      walk_flush<Batched>(W.ncols);
       const bool more = W.more != 0u;
       __syncwarp();
       if (lane == 0u) {
@@ -749,8 +781,8 @@ __device__ __noinline__ uint32_t walk_manage(const uint32_t round, uint32_t sp, 
 // until a round hands nothing over.
 template <bool Batched>
 __global__ void __launch_bounds__(kWalkThreads, kWalkBlocksPerSm) k_walk(const __grid_constant__ WalkArgs w) {
-  WalkSmem& S = walk_shared();
-  WalkWarp& W = walk_warp();
+  WalkSmem<Batched>& S = walk_shared<Batched>();
+  WalkWarp<Batched>& W = walk_warp<Batched>();
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt = (1u << lane) - 1u;
   for (uint32_t i = threadIdx.x; i < (uint32_t)kZigLayers; i += blockDim.x)
@@ -782,7 +814,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkBlocksPerSm) k_walk(const _
 #pragma unroll 1
       do {
         if (walk_step<Batched, true>(w.a.ks, S, W, lane, lt, sp, np) && np >= 32u) left = 1u;
-      } while (--left != 0u && sp - 32u <= kStackRoom - 32u);
+      } while (--left != 0u && sp - 32u <= kStackRoom<Batched> - 32u);
       steps = kPollSteps - left;
     }
     __syncwarp();
