@@ -674,7 +674,15 @@ __device__ __noinline__ uint32_t walk_load(uint32_t round, uint32_t sp) {
   }
   const uint32_t n = min(lend, h.w + h.y) - lpos;  // at most 32
   if (lane < n) {
-    uint4 e = __ldcg(w.region[old] + (uint64_t)h.x * w.region_stride + (lpos - h.w) + lane);
+    // A stack's cells grow shallower, with larger trees, towards its bottom, so a supply takes
+    // every m-th cell: the source's cells j, j + m, ... for j = 0, then 1, ... (32 neighbours
+    // instead: 7.7e8 divisions of 256 instances 7.9 ms and 8 rounds against 6.5 and 6, 3.9e7
+    // divisions of 1e5 initial cells 0.55 against 0.45 ms.)
+    const uint32_t m = (h.y + 31u) / 32u, a = h.y / m, b = h.y % m;
+    const uint32_t p = lpos - h.w + lane;
+    const uint32_t j = p < b * (a + 1u) ? p / (a + 1u) : (p - b) / a;
+    const uint32_t i = j + (p - j * a - min(j, b)) * m;
+    uint4 e = __ldcg(w.region[old] + (uint64_t)h.x * w.region_stride + i);
     e.w += shared_address(W.window) + 4u * kColWords * ncols + (ncols << kMetaColShift);
     stack_put(W, sp + lane, e);
   }
