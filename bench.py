@@ -47,6 +47,7 @@ sys.path.insert(0, PKG)
 METRIC = "cell divisions/s"
 UNIT = "divisions/s"
 ALG_BYTES_PER_NODE = 32  # 16-byte cell state written once and read once per tree node
+DEFAULT_CONFIG = 4  # the configuration that runs as a tree walk where it can
 FP64_OPS_PER_DIVISION = 4  # per daughter: tau = fma(sd, z, mean) and due = birth + tau
 
 
@@ -242,6 +243,55 @@ def reference_batched_line(steps, warmup, per_step):
     return line
 
 
+def profiled(name):
+    """The number at the start of a summary in profiles/, or None."""
+    try:
+        with open(os.path.join(ROOT, "profiles", name)) as fh:
+            return float(fh.read().split()[0])
+    except (OSError, ValueError, IndexError):
+        return None
+
+
+def walk_roofline(ipd, divisions, ms, sms, clk, traffic, launches_per_step, sweep_gbs):
+    """Roofline of a run as a tree walk: warp instructions (ncu, profiles/) against the issue slots."""
+    peak = 4.0 * sms * clk["sm_mhz"] * 1e6 if clk.get("sm_mhz") else None
+    rate = ipd * divisions / (ms * 1e-3) if (ipd and ms > 0) else None
+    return {"bound": "issue", "achieved": rate, "peak": peak, "unit": "warp instructions/s",
+            "frac": (rate / peak) if (rate and peak) else None,
+            "traffic": traffic, "peak_source": "4 issue slots x %d SMs x sampled SM clock" % sms,
+            "kernel": "k_walk", "launches_per_step": launches_per_step, "sweep_alg_gbs": sweep_gbs,
+            "note": "%s warp instructions per division (ncu, profiles/k_walk.md); the cells stay in shared memory, so "
+                    "the launch has next to no DRAM traffic; sweep_alg_gbs is what a level sweep would have to move "
+                    "at this rate (64 B per division)" % ipd}
+
+
+def sweep_roofline(achieved, hbm, traffic, peak_kind, launches, divide_ms, steps, alg_bytes, fp64_rate, fp64_peak,
+                   issue_frac, ipd, sms, persistent):
+    """Roofline of a run by level sweeps: algorithmic bytes against HBM, with the FP64 pipe and issue."""
+    return {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
+            "frac": (achieved / hbm) if achieved else None, "traffic": traffic,
+            "peak_source": peak_kind,
+            "dram_achieved": (traffic * launches / (divide_ms * 1e-3) / 1e9)
+            if (traffic and divide_ms > 0) else None,
+            "dram_frac": (traffic * launches / (divide_ms * 1e-3) / 1e9 / hbm)
+            if (traffic and divide_ms > 0) else None,
+            "kernel": "k_persist" if persistent else "k_divide",
+            "launches_per_step": launches / steps,
+            "alg_bytes_per_launch": alg_bytes / launches,
+            "fp64_achieved": fp64_rate, "fp64_peak": fp64_peak,
+            "fp64_frac": (fp64_rate / fp64_peak) if (fp64_rate and fp64_peak) else None,
+            "fp64_unit": "FP64 lane-ops/s (%d per division; peak: pc_debug_peak FMA probe)"
+                         % FP64_OPS_PER_DIVISION,
+            "issue_frac": issue_frac,
+            "issue_note": "%s warp instructions per division (ncu, profiles/) x divisions / "
+                          "(4 x %d SMs x sampled SM clock)" % (ipd, sms),
+            "note": "alg bytes = 64 B per division (two 16-B nodes written+read); the "
+                    "kernel stores only daughters that divide again, so its DRAM traffic "
+                    "(dram_achieved, from the ncu bytes per division in profiles/) is about "
+                    "half of that and the sweep is bound by instruction issue, not HBM"
+                    + ("; the persistent launch also runs the root sweep" if persistent else "")}
+
+
 def run_ours(args):
     import numpy as np
     import torch
@@ -287,7 +337,9 @@ def run_ours(args):
         if world > 1:
             torch.distributed.barrier()
 
+    flush = torch.empty(1 << 28, dtype=torch.uint8, device="cuda")  # larger than the 129 MB L2
     for _ in range(args.warmup):
+        flush.zero_()
         plan.run()
     barrier()
     clocks = ClockSampler(local)
@@ -298,6 +350,7 @@ def run_ours(args):
     divide_ms = device_ms = 0.0
     e0.record(stream)
     for _ in range(args.steps):
+        flush.zero_()  # inside the timed region
         plan.run()
         reduce_counts()
         st = plan.stats()
@@ -352,37 +405,33 @@ def run_ours(args):
         return 0
 
     hbm, peak_kind = peaks()
-    # dominant kernel: the division sweep. Algorithmic bytes: each division creates two
-    # tree nodes, each node's 16-byte state written once and read once (32 B per node).
+    # dominant kernel: the tree walk (default configuration), or the division sweep. Algorithmic
+    # bytes of the sweep: each division creates two tree nodes, each node's 16-byte state written
+    # once and read once (32 B per node).
     alg_bytes = 2 * ALG_BYTES_PER_NODE * divisions
     persistent = bool(tuning and tuning["driver"])
-    launches = max(1, args.steps if persistent else sweeps)  # launches of the dominant kernel
+    walks = (tuning["config"] if tuning else DEFAULT_CONFIG) == DEFAULT_CONFIG
+    launches = max(1, args.steps if persistent or walks else sweeps)  # launches of the dominant kernel
     achieved = alg_bytes / (divide_ms * 1e-3) / 1e9 if divide_ms > 0 else None
-    traffic = None
-    tpath = os.path.join(ROOT, "profiles", "traffic_per_division_persistent.txt" if persistent
-                         else "traffic_per_division.txt")
-    if os.path.exists(tpath):
-        try:
-            per_div = float(open(tpath).read().split()[0])
-            traffic = per_div * divisions / launches
-        except (ValueError, IndexError):
-            traffic = None
+    per_div = profiled("traffic_per_division_walk.txt" if walks else "traffic_per_division_persistent.txt" if persistent
+                       else "traffic_per_division.txt")
+    traffic = per_div * divisions / launches if per_div is not None else None
     # the division sweep's other ceilings: the FP64 pipe (two FMA + two adds per division,
     # the daughters' exact due times) against its measured peak, and instruction issue
     # (warp instructions per division from the ncu summary in profiles/) against four
     # issue slots per SM per cycle at the sampled SM clock
     fp64_peak = eng.peak("fp64")
     sms = torch.cuda.get_device_properties(local).multi_processor_count
-    ipd = None
-    try:
-        with open(os.path.join(ROOT, "profiles", "instructions_per_division.txt")) as fh:
-            ipd = float(fh.read().split()[0])
-    except (OSError, ValueError, IndexError):
-        pass
+    ipd = profiled("instructions_per_division_walk.txt" if walks else "instructions_per_division.txt")
     fp64_rate = FP64_OPS_PER_DIVISION * divisions / (divide_ms * 1e-3) if divide_ms > 0 else None
     issue_frac = None
     if ipd and divide_ms > 0 and clk.get("sm_mhz"):
         issue_frac = ipd * divisions / (divide_ms * 1e-3) / (4.0 * sms * clk["sm_mhz"] * 1e6)
+    if walks:
+        roofline = walk_roofline(ipd, divisions, divide_ms, sms, clk, traffic, launches / args.steps, achieved)
+    else:
+        roofline = sweep_roofline(achieved, hbm, traffic, peak_kind, launches, divide_ms, args.steps, alg_bytes,
+                                  fp64_rate, fp64_peak, issue_frac, ipd, sms, persistent)
     cpu = None
     if not args.no_cpu_baseline and world == 1:
         sys.path.insert(0, os.path.join(ROOT, "oracle"))
@@ -411,36 +460,14 @@ def run_ours(args):
         "data": "synthetic (seeded generator, procell/configs.py)",
         "config": {"workload": describe(w), "divisions_per_step": divisions // args.steps,
                    "nodes_per_step": (roots + 2 * divisions) // args.steps,
-                   "l2": "no flush: each step streams %.0f GB of level buffers, >> 129 MB L2"
-                         % (2 * 16 * divisions / args.steps / 1e9),
+                   "l2": "flushed before each step (a 268 MB buffer written, inside the timed region)",
                    "parallelism": (f"one input, initial cells split over {world} GPUs by expected work, "
                                    f"one all_reduce of the counts per step" if roots_split
                                    else f"one independent instance per GPU x{world}"),
                    "tuning": tuning},
         "e2e": {"value": tot_e2e_div / e2e_t, "unit": UNIT,
                 "h2d_bytes_per_step": h2d // args.steps, "d2h_bytes_per_step": d2h // args.steps},
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
-                     "frac": (achieved / hbm) if achieved else None, "traffic": traffic,
-                     "peak_source": peak_kind,
-                     "dram_achieved": (traffic * launches / (divide_ms * 1e-3) / 1e9)
-                     if (traffic and divide_ms > 0) else None,
-                     "dram_frac": (traffic * launches / (divide_ms * 1e-3) / 1e9 / hbm)
-                     if (traffic and divide_ms > 0) else None,
-                     "kernel": "k_persist" if (tuning and tuning["driver"]) else "k_divide",
-                     "launches_per_step": launches / args.steps,
-                     "alg_bytes_per_launch": alg_bytes / launches,
-                     "fp64_achieved": fp64_rate, "fp64_peak": fp64_peak,
-                     "fp64_frac": (fp64_rate / fp64_peak) if (fp64_rate and fp64_peak) else None,
-                     "fp64_unit": "FP64 lane-ops/s (%d per division; peak: pc_debug_peak FMA probe)"
-                                  % FP64_OPS_PER_DIVISION,
-                     "issue_frac": issue_frac,
-                     "issue_note": "%s warp instructions per division (ncu, profiles/) x divisions / "
-                                   "(4 x %d SMs x sampled SM clock)" % (ipd, sms),
-                     "note": "alg bytes = 64 B per division (two 16-B nodes written+read); the "
-                             "kernel stores only daughters that divide again, so its DRAM traffic "
-                             "(dram_achieved, from the ncu bytes per division in profiles/) is about "
-                             "half of that and the sweep is bound by instruction issue, not HBM"
-                             + ("; the persistent launch also runs the root sweep" if persistent else "")},
+        "roofline": roofline,
         "gpu_launches": kernels,
         "clocks": clk,
         "device_ms_per_step": device_ms / args.steps,
@@ -556,7 +583,7 @@ def measure_batched(eng, local, steps, warmup, tune, cpu_seconds, e2e_steps):
     elapsed_ms = e0.elapsed_time(e1)
     # the same batch as one persistent cooperative launch per run, replayed from a CUDA graph
     # (the autotuner keeps whichever driver is faster; both are reported)
-    cfg_sel = tuning["config"] if tuning else 4
+    cfg_sel = tuning["config"] if tuning else DEFAULT_CONFIG
     eng.set_option("sweep_config", cfg_sel)
     eng.set_option("driver", 1)
     eng.set_option("graph", 1)
@@ -628,7 +655,8 @@ def measure_batched(eng, local, steps, warmup, tune, cpu_seconds, e2e_steps):
     hbm, peak_kind = peaks()
     alg_bytes = 2 * ALG_BYTES_PER_NODE * divisions
     persistent = bool(tuning and tuning["driver"])
-    launches = max(1, steps if persistent else sweeps)
+    walks = cfg_sel == DEFAULT_CONFIG
+    launches = max(1, steps if persistent or walks else sweeps)
     achieved = alg_bytes / (divide_ms * 1e-3) / 1e9 if divide_ms > 0 else None
     value = n * steps / (elapsed_ms * 1e-3)
     e2e_value = n * e2e_steps / e2e_t
@@ -654,8 +682,10 @@ def measure_batched(eng, local, steps, warmup, tune, cpu_seconds, e2e_steps):
                    "divisions_per_step": divisions // steps,
                    "nodes_per_step": (roots + 2 * divisions) // steps,
                    "tuning": tuning,
-                   "l2": "no flush: each step streams %.0f GB of level buffers, >> 129 MB L2"
-                         % (2 * 16 * divisions / steps / 1e9)},
+                   "l2": ("no flush: the inputs are a few MB and the walk keeps its cells in shared memory; bound by "
+                          "instruction issue" if walks else
+                          "no flush: each step streams %.0f GB of level buffers, >> 129 MB L2"
+                          % (2 * 16 * divisions / steps / 1e9))},
         "divisions_per_s": divisions / (elapsed_ms * 1e-3),
         "loop_plain": {"run_instances_per_s": n / loop_run_s,
                        "e2e_instances_per_s": n / loop_e2e_s,
@@ -672,8 +702,12 @@ def measure_batched(eng, local, steps, warmup, tune, cpu_seconds, e2e_steps):
         "bit_exact_instances": "%d/%d" % (same, n),
         "e2e": {"value": e2e_value, "unit": "instances/s", "h2d_bytes_per_step": h2d // e2e_steps,
                 "d2h_bytes_per_step": d2h // e2e_steps, "steps": e2e_steps},
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
-                     "frac": (achieved / hbm) if achieved else None, "traffic": batched_traffic(divisions, launches),
+        "roofline": walk_roofline(profiled("instructions_per_division_walk_batched.txt"), divisions, divide_ms,
+                                  torch.cuda.get_device_properties(local).multi_processor_count, clk,
+                                  batched_traffic(divisions, launches, walks), launches / steps, achieved) if walks else
+                    {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
+                     "frac": (achieved / hbm) if achieved else None,
+                     "traffic": batched_traffic(divisions, launches, walks),
                      "peak_source": peak_kind, "kernel": "k_persist" if persistent else "k_divide",
                      "launches_per_step": launches / steps,
                      "alg_bytes_per_launch": alg_bytes / launches},
@@ -963,14 +997,10 @@ def measure_calibration(eng, local, steps, warmup, cpu_seconds, pso_seconds, ext
     return line
 
 
-def batched_traffic(divisions, launches):
-    """Measured DRAM bytes per division of the batched sweeps (ncu, profiles/) x divisions
-    per launch."""
-    try:
-        with open(os.path.join(ROOT, "profiles", "traffic_per_division_batched.txt")) as fh:
-            return float(fh.read().split()[0]) * divisions / max(1, launches)
-    except (OSError, ValueError, IndexError):
-        return None
+def batched_traffic(divisions, launches, walks):
+    """Measured DRAM bytes per division of a batched run (ncu, profiles/) x divisions per launch."""
+    per_div = profiled("traffic_per_division_walk_batched.txt" if walks else "traffic_per_division_batched.txt")
+    return per_div * divisions / max(1, launches) if per_div is not None else None
 
 
 def cpu_batched_sample(instances, seconds):

@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(256) k_merge_counts(const unsigned long long* 
 
 // Every instance's merged totals from a batch's count table, one thread per (generation, bin):
 // a pass over the table (the floor) with one atomic per nonzero sum. 256 instances of 256 bins
-// and 3 types, 14 generations (22 MB): reading the totals of a run takes 0.27 ms, most of it
+// and 3 types, 14 generations (22 MB): reading the totals of a run takes 0.33 ms, most of it
 // the 3.8 MB back; the table back and a host merge took 0.99 ms.
 __global__ void __launch_bounds__(256) k_merge_totals(const unsigned long long* __restrict__ h, uint64_t nclass,
                                                       const MergeInstance* __restrict__ inst,

@@ -55,9 +55,9 @@ constexpr uint32_t kBudget = 1u << 16;
 // Resident blocks per SM the lineage-walk kernels are compiled for (registers per thread =
 // 65536 / (128 x this)); compile-time tuning, results do not depend on it. Drawing in every
 // pass (calibration input, one walk per lane): 5 blocks forward 1.91, adjoint 2.62 ms; 6 1.75 /
-// 2.45; 8 3.04 / 2.45. Kept draws, two walks per lane, 256 candidates: forward 8 blocks 0.782,
-// 7 0.778, 6 0.831, 5 0.824 ms; Jacobian 7 0.916, 6 0.909, 5 0.912, 4 0.947; adjoint 6 (all its
-// shared memory allows) 0.979, 5 1.048.
+// 2.45; 8 3.04 / 2.45. Kept draws, two walks per lane, 256 candidates: forward 8 blocks 0.700,
+// 7 0.691, 6 0.712 ms; Jacobian 7 0.830, 6 0.810, 5 0.814; adjoint 6 (all its shared memory
+// allows) 0.862, 5 0.927.
 constexpr int kBlocksDrawn = 6;
 constexpr int kBlocksKept = 7;
 constexpr int kBlocksKeptJacobian = 6;
@@ -494,8 +494,9 @@ struct RemGrid2 {
 // form (relative errors near 2^-22 for |x| up to a few tens, and 2^-23). The intrinsics __expf and
 // __fdividef also serve subnormal results and any y, which costs instructions in every step and
 // which no pair needs: y is between 1 and 2, and a factor below 2^-126 takes its product below
-// the stopping level, which ends the walk (a bin has at most 64 steps, see stop_level). Forward 0.794 -> 0.691, adjoint 0.979 -> 0.862, Jacobian 0.910 -> 0.810 ms for 256
-// candidates (with the walk above left to add what is below the level, instead of 0).
+// the stopping level, which ends the walk (a bin has at most 64 steps, see stop_level). 256
+// candidates: forward 0.794 -> 0.691, adjoint 0.979 -> 0.862, Jacobian 0.910 -> 0.810 ms (with a
+// walk below that level left to add its last weights, instead of set to 0 in each step).
 __device__ __forceinline__ float exp_neg(float x) {
   float e;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__fmul_rn(-fabsf(x), 1.4426950408889634f)));
