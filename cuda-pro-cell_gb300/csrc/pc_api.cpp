@@ -519,11 +519,11 @@ class ResultMemory {
       const size_t size = it->first;
       kept_.erase(it);
       kept_bytes_ -= size;
-      out_[p] = size;
+      note(p, size);
       return p;
     }
     void* p = std::malloc(bytes);
-    if (p) out_[p] = bytes;
+    if (p) note(p, bytes);
     return p;
   }
   // Pinned memory for the device to write a result's counts into directly (copying 7 MB out of
@@ -585,9 +585,12 @@ class ResultMemory {
     const size_t size = it->second;
     out_.erase(it);
     if (kept_bytes_ + size <= kKept) {
-      kept_.emplace(size, p);
-      kept_bytes_ += size;
-      return;
+      try {
+        kept_.emplace(size, p);
+        kept_bytes_ += size;
+        return;
+      } catch (...) {  // not kept
+      }
     }
     lock.unlock();
     std::free(p);
@@ -595,6 +598,13 @@ class ResultMemory {
 
  private:
   static constexpr size_t kSmall = size_t(64) << 10, kKept = size_t(64) << 20;
+  // An array whose size could not be noted is freed instead of kept.
+  void note(void* p, size_t size) {
+    try {
+      out_[p] = size;
+    } catch (...) {
+    }
+  }
   std::mutex m_;
   std::multimap<size_t, void*> kept_;
   std::map<void*, size_t> out_;
@@ -1964,7 +1974,12 @@ bool walk_serves(const pc_context* ctx, const pc_plan* p) {
 int enqueue_walk(pc_context* ctx, pc_plan* p, const WalkArgs& w, int grid, cudaStream_t s) {
   // the control words lie behind the counts: one clear for both
   PC_CUDA(ctx, pc_cuda_memset(p->hist_dev, 0, p->hist_elems * sizeof(unsigned long long) + sizeof(WalkCtl), s));
-  PC_CUDA(ctx, PC_LAUNCH(launch_walk(w, grid, s)));
+  const cudaError_t e = PC_LAUNCH(launch_walk(w, grid, s));
+  if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs at hand than the device has
+    (void)cudaGetLastError();
+    return PC_ERR_UNSUPPORTED;
+  }
+  PC_CUDA(ctx, e);
   PC_CUDA(ctx, pc_cuda_copy(ctx->pinned + 24, w.ctl, offsetof(WalkCtl, barrier), cudaMemcpyDeviceToHost, s));
   return PC_OK;
 }
@@ -1978,7 +1993,8 @@ int run_walk(pc_context* ctx, pc_plan* p, const RunArgs& a) {
     int n = 0;
     const int e = walk_occupancy(p->batched, &n);
     if (e != 0) return fail(ctx, PC_ERR_CUDA, std::string("occupancy query: ") + cudaGetErrorString((cudaError_t)e));
-    occ = std::max(1, n);
+    if (n == 0) return PC_ERR_UNSUPPORTED;
+    occ = n;
   }
   const int grid = max_blocks(ctx, occ);
   const uint64_t nroots = p->root_end - p->root_begin;
@@ -2011,7 +2027,11 @@ int run_walk(pc_context* ctx, pc_plan* p, const RunArgs& a) {
     pc_cuda_free(ctx->walk_dev);
     ctx->walk_dev = nullptr;
     ctx->walk_bytes = 0;
-    PC_CUDA(ctx, pc_cuda_malloc(&ctx->walk_dev, need));
+    if (pc_cuda_malloc(&ctx->walk_dev, need) != cudaSuccess) {  // the level sweeps make do with less
+      (void)cudaGetLastError();
+      ctx->walk_dev = nullptr;
+      return PC_ERR_UNSUPPORTED;
+    }
     ctx->walk_bytes = need;
   }
   char* at = static_cast<char*>(ctx->walk_dev);

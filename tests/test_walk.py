@@ -163,3 +163,31 @@ def test_batch_of_every_case_and_mixed_with_a_deep_one(engine, oracle_lib):
         for i, n in enumerate(names):
             o = oracle_lib.simulate(*CASES[n][:3], 1.0, seed=100 + i, nthreads=0)
             assert np.array_equal(got[i].per_type, o.per_type), n
+
+
+@pytest.mark.gpu
+def test_a_walk_without_scratch_goes_to_the_level_sweeps(oracle_lib):
+    """Every CUDA call of a context's first run failed in turn: an error status or exact counts,
+    and for one of them (the walk's scratch) the level sweeps give them."""
+    import procell.configs as cfg
+    from procell import Engine, ProcellError
+    w = cfg.small()
+    o = oracle_lib.simulate(w.bins, w.types, w.t_max, w.phi, seed=w.seed, nthreads=0)
+    by_sweeps, n = 0, 1
+    while True:
+        eng = Engine(0)
+        try:
+            f0 = eng.get_option("faults_injected")
+            eng.set_option("fail_nth_call", n)
+            try:
+                r = eng.simulate(w.bins, w.types, w.t_max, w.phi, w.seed)
+                assert np.array_equal(r.per_type, o.per_type)
+                by_sweeps += r.stats["kernel_launches"] > 1
+            except ProcellError as e:
+                assert e.code in (2, 3), n  # PC_ERR_CUDA, PC_ERR_NOMEM
+            if eng.get_option("faults_injected") == f0:  # past the run's last call
+                break
+        finally:
+            eng.close()
+        n += 1
+    assert n > 5 and by_sweeps == 1
