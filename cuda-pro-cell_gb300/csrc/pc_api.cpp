@@ -2876,6 +2876,8 @@ SmoothArgs smooth_args(const pc_context* ctx, const pc_smooth* s) {
   A.ncells = (uint32_t)s->I.roots;
   A.t_max = s->I.t_max;
   A.inv_h = 1.0 / s->h;
+  A.h = 1.0 / A.inv_h;
+  A.inv_paths = 1.0 / (double)s->paths;
   A.bin_start = s->bin_start_dev;
   A.bin_cap = s->bin_cap_dev;
   A.bin_order = s->bin_cap_dev + s->I.bin_value.size();

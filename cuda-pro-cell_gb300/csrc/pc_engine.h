@@ -272,7 +272,7 @@ struct SmoothArgs {
   uint32_t nbins, rows;       // rows = max cap + 1 (generation rows per bin)
   uint32_t ntypes, paths;     // lineages sampled per initial cell (independent replicas)
   uint32_t ncells;            // initial cells; replica m of cell r draws as cell r + m * ncells
-  double t_max, inv_h;
+  double t_max, inv_h, h, inv_paths;  // h as 1 / inv_h
   const uint64_t* bin_start;  // [nbins + 1]
   const uint32_t* bin_cap;    // [nbins]
   const uint32_t* bin_order;  // [nbins] the bins in launch order (most expensive first)

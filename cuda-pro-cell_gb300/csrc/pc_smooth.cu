@@ -57,7 +57,7 @@ constexpr uint32_t kBudget = 1u << 16;
 // pass (calibration input, one walk per lane): 5 blocks forward 1.91, adjoint 2.62 ms; 6 1.75 /
 // 2.45; 8 3.04 / 2.45. Kept draws, two walks per lane, 256 candidates: forward 8 blocks 0.700,
 // 7 0.691, 6 0.712 ms; Jacobian 7 0.830, 6 0.810, 5 0.814; adjoint 6 (all its shared memory
-// allows) 0.862, 5 0.927.
+// allows) 0.862, 5 0.927 (before grid_shared).
 constexpr int kBlocksDrawn = 6;
 constexpr int kBlocksKept = 7;
 constexpr int kBlocksKeptJacobian = 6;
@@ -69,6 +69,13 @@ __device__ __forceinline__ double f32_to_f64_bits(float z) {
   const uint32_t hi = (f & 0x80000000u) | (a ? (a >> 3) + (896u << 20) : 0u);
   return __hiloint2double((int)hi, (int)(f << 29));
 }
+// (double)x for any float, and 2^e for normal results, off the FP64 pipe.
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t a = __float_as_uint(x) & 0x7FFFFFFFu;
+  if (a - 1u >= 0x7F7FFFFFu || a < 0x00800000u) return a == 0u ? 0.0 : (double)x;  // subnormal, infinite or NaN
+  return f32_to_f64_bits(x);
+}
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 
 __device__ __noinline__ float node_z_slow(uint32_t j, uint32_t layer, uint32_t wedge, uint64_t node, uint32_t root,
                                           uint32_t k0, uint32_t k1, const ZigTables& Z, uint32_t* error) {
@@ -221,11 +228,12 @@ __device__ __forceinline__ bool grid_setup(RemGrid& r, double mu, double sigma, 
   int e;
   frexp(B, &e);  // B < 2^e
   const int m = e + 1;
-  const double g = ldexp(1.0, m - 23);
+  const double g = pow2(m - 23);
   if (!(g * (double)steps * (double)steps <= 16.0 * h) || m > 100) return false;
-  const double mu_g = ldexp(rint(ldexp(mu, 23 - m)), m - 23);
-  const double t_g = ldexp(rint(ldexp(t_max, 23 - m)), m - 23);
-  r.C = (float)ldexp(1.5, m);
+  const double inv_g = pow2(23 - m);
+  const double mu_g = rint(mu * inv_g) * g;
+  const double t_g = rint(t_max * inv_g) * g;
+  r.C = __uint_as_float(((uint32_t)(127 + m) << 23) | 0x400000u);  // 1.5 * 2^m
   r.mu_g = (float)mu_g;
   r.mu_f = (float)(mu - mu_g);
   r.sg_h = (float)sigma;
@@ -234,6 +242,37 @@ __device__ __forceinline__ bool grid_setup(RemGrid& r, double mu, double sigma, 
   r.t_f = (float)(t_max - t_g);
   r.Rh = r.Rl = 0.0f;
   return true;
+}
+
+// grid_setup of a block's 32 candidates by its first warp, for all of them: seven floats per
+// candidate through the start of `scratch` (the block's draws overwrite it only after the second
+// barrier). C = 0 stands for false. With the set-up done by every warp, powers of two by ldexp and
+// the sums widened by conversions, a third of the FP64 pipe's time went there: Jacobian 0.810 ->
+// 0.790 ms for 256 candidates, 0.163 -> 0.157 for 37 of 97 bins, forward 0.691 -> 0.686 ms.
+__device__ __forceinline__ bool grid_shared(RemGrid& r, double mu, double sigma, double t_max, uint32_t steps, double h,
+                                            float* scratch) {
+  float* const s = scratch + (threadIdx.x & 31u);
+  if (threadIdx.x < 32u) {
+    if (!grid_setup(r, mu, sigma, t_max, steps, h)) r.C = 0.0f;
+    s[0] = r.C;
+    s[32] = r.mu_g;
+    s[64] = r.mu_f;
+    s[96] = r.sg_h;
+    s[128] = r.sg_l;
+    s[160] = r.t_g;
+    s[192] = r.t_f;
+  }
+  __syncthreads();
+  r.C = s[0];
+  r.mu_g = s[32];
+  r.mu_f = s[64];
+  r.sg_h = s[96];
+  r.sg_l = s[128];
+  r.t_g = s[160];
+  r.t_f = s[192];
+  r.Rh = r.Rl = 0.0f;
+  __syncthreads();
+  return r.C != 0.0f;
 }
 
 // A lineage stops once no later generation can add more than e^-40 cells: every later leaf
@@ -660,13 +699,12 @@ __global__ void __launch_bounds__(kThreads, Kept ? kBlocksKeptJacobian : kBlocks
     sd = params[(uint64_t)c * KQ + 3u * k + 2u];
   }
   const bool quiescent = neg_nonzero(mu), fixed_tau = zero_bits(mu);
-  __syncthreads();
   const uint32_t steps = __ldg(A.bin_cap + b) + 1u;
   const uint64_t r0 = __ldg(A.bin_start + b), r1 = __ldg(A.bin_start + b + 1);
   float* fmy = facc + threadIdx.x;
   const float inv_h = (float)A.inv_h;
   RemGrid rg;
-  const bool grid = opaque(grid_setup(rg, mu, sd, A.t_max, steps, 1.0 / A.inv_h));
+  const bool grid = opaque(grid_shared(rg, mu, sd, A.t_max, steps, A.h, reinterpret_cast<float*>(u_age)));
   const RemFp64 rd{mu, sd, A.t_max, 0.0};
   const bool pairs = opaque(grid && !quiescent && !fixed_tau);
   const RemGrid2 rg2(rg, rg);
@@ -702,13 +740,13 @@ __global__ void __launch_bounds__(kThreads, Kept ? kBlocksKeptJacobian : kBlocks
   // sums over the warps in warp order, generation g's rows scaled by 2^g; lane l of every
   // warp holds candidate 32 * group + l, so the warps split the rows
   if (!live) return;
-  const double inv_paths = 1.0 / (double)A.paths;
+  const double inv_paths = A.inv_paths;
   double* o = out + ((uint64_t)c * A.nbins + b) * A.rows * KQ + 3u * k;
   for (uint32_t q = warp; q < 3u * A.rows; q += kWarps) {
     double v = 0.0;
 #pragma unroll
-    for (uint32_t w = 0; w < kWarps; ++w) v += (double)facc[q * kThreads + w * 32u + lane];
-    o[(q / 3u) * KQ + q % 3u] = ldexp(v * (q % 3u == 0u ? 1.0 : ratio) * inv_paths, (int)(q / 3u));
+    for (uint32_t w = 0; w < kWarps; ++w) v += widen(facc[q * kThreads + w * 32u + lane]);
+    o[(q / 3u) * KQ + q % 3u] = v * (q % 3u == 0u ? 1.0 : ratio) * inv_paths * pow2((int)(q / 3u));
   }
 }
 
@@ -763,13 +801,12 @@ __global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoin
   const bool quiescent = neg_nonzero(mu), fixed_tau = zero_bits(mu);
   // a type of ratio 0 adds nothing to the expected counts (its adjoint rows still count)
   const bool walks = Backward || (live && !zero_bits(my_prm[0]));
-  __syncthreads();
   const uint64_t r0 = __ldg(A.bin_start + b), r1 = __ldg(A.bin_start + b + 1);
   float* fmy = facc + threadIdx.x;
   const float inv_h = (float)A.inv_h;
   const float* my_ag = Backward ? Ag2 + lane : nullptr;
   RemGrid rg;
-  const bool grid = opaque(grid_setup(rg, mu, sd, A.t_max, steps, 1.0 / A.inv_h));
+  const bool grid = opaque(grid_shared(rg, mu, sd, A.t_max, steps, A.h, reinterpret_cast<float*>(u_age)));
   const RemFp64 rd{mu, sd, A.t_max, 0.0};
   const bool pairs = opaque(grid && walks && !quiescent && !fixed_tau);
   const RemGrid2 rg2(rg, rg);
@@ -832,7 +869,7 @@ __global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoin
   // rows by 1 / paths, and those of mean and sd by the ratio); lane l of every warp holds
   // candidate 32 * group + l, so the warps split the rows
   if (!live) return;
-  const double inv_paths = 1.0 / (double)A.paths, ratio = my_prm[0];
+  const double inv_paths = A.inv_paths, ratio = my_prm[0];
   const uint32_t nrows = Backward ? 3u : A.rows;
   double* o = Backward ? out + ((uint64_t)c * A.nbins + b) * KQ + 3u * k
                        : out + (((uint64_t)c * A.ntypes + k) * A.nbins + b) * A.rows;
@@ -840,11 +877,11 @@ __global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoin
     double v = 0.0;
 #pragma unroll
     for (uint32_t w = 0; w < kWarps; ++w)
-      v += (double)facc[2 * q * kThreads + w * 32u + lane] - (double)facc[(2 * q + 1) * kThreads + w * 32u + lane];
+      v += widen(facc[2 * q * kThreads + w * 32u + lane]) - widen(facc[(2 * q + 1) * kThreads + w * 32u + lane]);
     if constexpr (Backward)
       v *= (q == 0u ? 1.0 : ratio) * inv_paths;
     else
-      v *= ldexp(ratio * inv_paths, (int)q);
+      v *= ratio * inv_paths * pow2((int)q);
     o[q] = v;
   }
 }
