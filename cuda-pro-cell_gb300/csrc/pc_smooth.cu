@@ -675,8 +675,9 @@ __device__ __forceinline__ uint32_t candidate_of(const SmoothArgs& A, uint32_t n
 template <bool Kept>
 __global__ void __launch_bounds__(kThreads, Kept ? kBlocksKeptJacobian : kBlocksDrawn) k_smooth_jacobian(const SmoothArgs A, const double* __restrict__ params,
                                                               uint32_t ncand, double* __restrict__ out) {
-  // dynamic: per-thread sums [3 * rows][kThreads], then the lineage draws [kWarps][rows][32]
-  extern __shared__ float facc[];
+  // dynamic: per-thread sums [3 * rows][kThreads], then the lineage draws [kWarps][rows][32],
+  // read two floats at a time (a float's alignment would leave it to the static arrays' size)
+  extern __shared__ __align__(16) float facc[];
   __shared__ typename std::conditional<Kept, uint32_t, ZigTables>::type Z;  // kept draws need no tables
   __shared__ double u_age[kThreads];
   __shared__ __align__(8) float u_one[kThreads], u_one_lo[kThreads];
@@ -759,8 +760,8 @@ __global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoin
                                                      uint32_t nvalues, const int32_t* __restrict__ vidx,
                                                      double* __restrict__ out) {
   // dynamic: compensated FP32 accumulator pairs [arows][kThreads] (forward: 2 per generation
-  // row, backward: 2 per parameter), then the lineage draws z [kWarps][rows][32]
-  extern __shared__ float facc[];
+  // row, backward: 2 per parameter), then the lineage draws z [kWarps][rows][32] (8-byte reads)
+  extern __shared__ __align__(16) float facc[];
   __shared__ typename std::conditional<Kept, uint32_t, ZigTables>::type Z;  // kept draws need no tables
   __shared__ double u_age[kThreads];
   __shared__ __align__(8) float u_one[kThreads], u_one_lo[kThreads];
@@ -1029,7 +1030,7 @@ __global__ void __launch_bounds__(kGnThreads) k_smooth_gauss_newton(
     const uint32_t* __restrict__ inv_off, const uint32_t* __restrict__ inv_idx, uint32_t nvalues,
     const double* __restrict__ target_log, double* __restrict__ loss, double* __restrict__ jtj,
     double* __restrict__ jtr) {
-  extern __shared__ double gsm[];  // [tile][kq + 1]: scaled Jacobian row, then r
+  extern __shared__ __align__(16) double gsm[];  // [tile][kq + 1]: scaled Jacobian row, then r
   const uint32_t c = blockIdx.x, tid = threadIdx.x;
   const uint32_t w = kq + 1u;
   const uint32_t nout = kq * (kq + 1u) / 2u + kq + 1u;
