@@ -783,6 +783,7 @@ __global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoin
   for (uint32_t i = 0; i < arows; ++i) facc[i * kThreads + threadIdx.x] = 0.0f;
   const uint32_t cap = __ldg(A.bin_cap + b);
   const uint32_t steps = cap + 1u;
+  bool finite = true;
   if constexpr (Backward) {
     for (uint32_t i = threadIdx.x; i < 32u * steps; i += blockDim.x) {
       const uint32_t g = i / 32u, sl = blockIdx.y * 32u + i % 32u;
@@ -793,7 +794,11 @@ __global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoin
         if (v >= 0) a = ldexp(grad_expected[(uint64_t)cc * nvalues + v], (int)g);
       }
       Ag2[i] = (float)a;
+      finite = finite && isfinite((float)a);
     }
+    // A gradient that is not finite (FP32) is left out where a weight is 0, which walk() looks
+    // for and a pair does not: the whole block walks alone.
+    finite = __syncthreads_and(finite) != 0;
   }
   const double* my_prm = params + (uint64_t)(live ? c : 0u) * KQ + 3u * k;
   const double mu = live ? my_prm[1] : 0.0, sd = live ? my_prm[2] : 0.0;
@@ -809,7 +814,7 @@ __global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoin
   RemGrid rg;
   const bool grid = opaque(grid_shared(rg, mu, sd, A.t_max, steps, A.h, reinterpret_cast<float*>(u_age)));
   const RemFp64 rd{mu, sd, A.t_max, 0.0};
-  const bool pairs = opaque(grid && walks && !quiescent && !fixed_tau);
+  const bool pairs = opaque(grid && walks && finite && !quiescent && !fixed_tau);
   const RemGrid2 rg2(rg, rg);
   const float stop = stop_level(steps);  // once per block: the walks' stopping threshold
   // lineage i of the bin: initial cell r0 + i / paths, replica i % paths

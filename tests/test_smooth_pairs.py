@@ -96,3 +96,46 @@ def test_gauss_newton_of_every_width(engine, types):
     assert torch.allclose(jtj, torch.einsum("cvp,cvq->cpq", Js, Js), rtol=1e-11, atol=1e-12 * float(jtj.abs().max()))
     assert torch.allclose(jtr, torch.einsum("cvp,cv->cp", Js, r), rtol=1e-11, atol=1e-12 * float(jtr.abs().max()))
     sm.close()
+
+
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 1e300])  # 1e300: infinite once in FP32
+def test_gradient_that_is_not_finite_where_no_cell_is(engine, bad):
+    """A loss may have an infinite or undefined gradient at an expected count of 0 (sqrt(E), xlogy);
+    a generation none of whose lineages has any weight adds nothing to the adjoint, whatever its
+    gradient, for even and odd numbers of lineages alike. The values of weight 0 are those of the
+    lineages walked alone. Tolerance as in test_pairs_against_single_walks."""
+    import torch
+    from procell.smooth import Smooth
+    depth, cand = 11, 64
+    v = 1.5 * 2.0 ** depth
+    rng = np.random.default_rng(8)
+    mean = np.exp(rng.uniform(np.log(8.0), np.log(70.0), cand))
+    P = torch.tensor(np.stack([np.ones(cand), mean, 0.5 * mean], 1)[:, None, :], device="cuda")
+    hit = 0
+    for lineages in (2, 3, 6):
+        apart = [v * (1.0 + i / 1024.0) for i in range(lineages)]
+        sm = Smooth(engine, [(a, 1) for a in apart], n_types=1, t_max=140.0, phi=1.0, h=0.5, paths=1, seed=23)
+        values = list(sm.values)
+        idx = np.array([[values.index(x / 2.0 ** g) for g in range(depth + 1)] for x in apart])
+        E, J = (x.cpu().numpy() for x in sm.jacobian(P))
+        sm.sync()
+        sm.close()
+        empty = E[:, idx].sum(1) == 0.0  # [candidate, generation]
+        terms = np.abs(J[:, idx]).sum(1)[:, :, 0]  # [candidate, generation, parameter]
+        sm = Smooth(engine, [(v, lineages)], n_types=1, t_max=140.0, phi=1.0, h=0.5, paths=1, seed=23)
+        values = list(sm.values)
+        at = np.array([values.index(v / 2.0 ** g) for g in range(depth + 1)])
+        gen_grad = rng.normal(size=depth + 1) * 0.5 ** np.arange(depth + 1)
+        got = []
+        for there in (0.0, bad):
+            grad = np.zeros((cand, sm.n_values))
+            grad[:, at] = np.where(empty, there, gen_grad)
+            got.append(sm.backward(P, torch.tensor(grad, device="cuda")).cpu().numpy()[:, 0])
+        sm.sync()
+        sm.close()
+        later = empty & (np.cumsum(~empty, 1) > 0) & (np.cumsum(~empty[:, ::-1], 1)[:, ::-1] > 0)
+        hit += int(later.any(1).sum())  # a generation of weight 0 between two others
+        tol = (64 * lineages + 2) * 2.0 ** -24 * np.einsum("g,cgq->cq", np.abs(gen_grad), terms) + 1e-10
+        assert np.all(np.isfinite(got[1]))
+        assert np.all(np.abs(got[1] - got[0]) <= tol)
+    assert hit > 0
