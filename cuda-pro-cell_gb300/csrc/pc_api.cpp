@@ -1318,20 +1318,33 @@ constexpr size_t kMaxMergeScratch = size_t(256) << 20;
 
 size_t round16(size_t n) { return (n + 15) & ~size_t(15); }
 
+// An allocation of the device merge that found no memory: the host merge makes do without.
+int merge_alloc(pc_context* ctx, cudaError_t e) {
+  if (e != cudaErrorMemoryAllocation) {
+    PC_CUDA(ctx, e);
+    return PC_OK;
+  }
+  (void)cudaGetLastError();
+  return PC_ERR_UNSUPPORTED;
+}
+
 // The device scratch and the pinned buffer of the merge, grown to at least these sizes.
 int ensure_merge(pc_context* ctx, size_t dev_bytes, size_t host_bytes) {
+  int rc = PC_OK;
   if (ctx->merge_dev_bytes < dev_bytes) {
     pc_cuda_free(ctx->merge_dev);
     ctx->merge_dev = nullptr;
     ctx->merge_dev_bytes = 0;
-    PC_CUDA(ctx, pc_cuda_malloc(&ctx->merge_dev, dev_bytes));
+    rc = merge_alloc(ctx, pc_cuda_malloc(&ctx->merge_dev, dev_bytes));
+    if (rc != PC_OK) return rc;
     ctx->merge_dev_bytes = dev_bytes;
   }
   if (ctx->merge_host_bytes < host_bytes) {
     cudaFreeHost(ctx->merge_host);
     ctx->merge_host = nullptr;
     ctx->merge_host_bytes = 0;
-    PC_CUDA(ctx, pc_cuda_malloc_host(&ctx->merge_host, host_bytes));
+    rc = merge_alloc(ctx, pc_cuda_malloc_host(&ctx->merge_host, host_bytes));
+    if (rc != PC_OK) return rc;
     ctx->merge_host_bytes = host_bytes;
   }
   return PC_OK;
@@ -1351,7 +1364,10 @@ size_t merge_map_bytes(const pc_plan* p) {
 int upload_map(pc_context* ctx, pc_plan* p, size_t bytes, uint64_t* uploaded) {
   *uploaded = 0;
   if (p->map_ready) return PC_OK;
-  if (!p->map_dev) PC_CUDA(ctx, take_spare(ctx->spare_map, bytes, &p->map_dev, &p->map_bytes));
+  if (!p->map_dev) {
+    const int rc = merge_alloc(ctx, take_spare(ctx->spare_map, bytes, &p->map_dev, &p->map_bytes));
+    if (rc != PC_OK) return rc;
+  }
   char* const h = reinterpret_cast<char*>(ctx->merge_host);
   const uint32_t n = (uint32_t)p->inst.size();
   std::vector<size_t> at(n + 1);
@@ -1395,7 +1411,7 @@ int upload_map(pc_context* ctx, pc_plan* p, size_t bytes, uint64_t* uploaded) {
 // The merged histogram of a single-instance plan, merged on the device from the count table
 // the run left there; the merged counts (values x (1 + types) u64) come back, instead of the
 // whole [generation][class] table and a host loop over it. Returns PC_ERR_UNSUPPORTED when
-// the scratch would exceed kMaxMergeScratch.
+// the scratch would exceed kMaxMergeScratch or cannot be allocated.
 int device_result(pc_context* ctx, pc_plan* p, pc_histogram* out) {
   const InstanceHost& I = p->inst[0];
   const uint32_t nb = (uint32_t)I.bin_value.size(), nt = (uint32_t)I.types.size();

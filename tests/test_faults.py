@@ -115,3 +115,38 @@ def test_every_failing_call_of_the_smoothed_form_is_reported(engine):
         assert np.array_equal(r[0], E0) and np.array_equal(r[1], G0)
 
     assert sweep_faults(engine, run, check) >= 4
+
+
+@pytest.mark.parametrize("batched", [False, True])
+def test_a_merge_without_memory_is_done_on_the_host(oracle_lib, small_oracle, batched):
+    """Every CUDA call of a context's first result failed in turn: an allocation of the device merge
+    that fails leaves the host merge, so none of them is reported as PC_ERR_NOMEM."""
+    from procell import Engine
+    w, o = small_oracle
+    recovered, n = 0, 1
+    while True:
+        eng = Engine(0)
+        try:
+            p = eng.batch([(w.bins, w.types, w.t_max, w.phi, w.seed)]) if batched else \
+                eng.plan(w.bins, w.types, w.t_max, w.phi, w.seed)
+            p.run()
+            live, f0 = eng.get_option("device_allocations"), eng.get_option("faults_injected")
+            eng.set_option("fail_nth_call", n)
+            try:
+                got = p.totals()[1] if batched else p.result().totals
+                assert np.array_equal(got, o.totals), n
+                recovered += int(eng.get_option("faults_injected") > f0)
+            except ProcellError as e:
+                assert e.code == PC_ERR_CUDA, (n, e)
+            done = eng.get_option("faults_injected") == f0
+            eng.set_option("fail_nth_call", 0)
+            got = p.totals()[1] if batched else p.result().totals
+            assert np.array_equal(got, o.totals), n
+            p.close()
+            assert eng.get_option("device_allocations") <= live + 2, n
+        finally:
+            eng.close()
+        if done:
+            break
+        n += 1
+    assert recovered >= 3  # scratch, pinned buffer, value map
