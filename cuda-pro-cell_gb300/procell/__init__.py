@@ -60,8 +60,9 @@ class Plan:
 
     def result(self) -> Result:
         h = (_lib.Histogram * 1)()
+        own = _lib.histogram_owners(h, 1)
         self.engine._check(self.engine.L.pc_plan_result(self.engine.ctx, self.handle, h))
-        return Result(*_lib.histograms_to_numpy(h, 1)[0])
+        return Result(*_lib.histograms_to_numpy(h, own)[0])
 
     def raw_counts(self) -> np.ndarray:
         L, n = self.engine.L, ctypes.c_uint64()
@@ -129,8 +130,9 @@ class Batch:
 
     def result(self, i: int) -> Result:
         h = (_lib.Histogram * 1)()
+        own = _lib.histogram_owners(h, 1)
         self.engine._check(self.engine.L.pc_batch_result(self.engine.ctx, self.handle, int(i), h))
-        return Result(*_lib.histograms_to_numpy(h, 1)[0])
+        return Result(*_lib.histograms_to_numpy(h, own)[0])
 
     def set_types(self, types):
         """New cell types for every instance: a TYPE_DTYPE array (or rows of (ratio, mean,
@@ -215,15 +217,17 @@ class Engine:
         arr, keep = instance_array(instances)
         n = len(instances)
         hs = (_lib.Histogram * max(1, n))()
+        own = _lib.histogram_owners(hs, n)
         self._check(self.L.pc_simulate_batch(self.ctx, arr, n, hs))
         del keep
-        return [Result(*r) for r in _lib.histograms_to_numpy(hs, n)]
+        return [Result(*r) for r in _lib.histograms_to_numpy(hs, own)]
 
     def simulate(self, bins, types, t_max, phi=None, seed=0, root_begin=None, root_end=None) -> Result:
         """pc_simulate (pc_simulate_shard for a range of initial cells): one input's merged
         histogram, host arrays in and out, in one library call."""
         b, t = _lib.bins_numpy(bins), _lib.types_numpy(types)
         h = (_lib.Histogram * 1)()
+        own = _lib.histogram_owners(h, 1)
         args = (self.ctx, b.ctypes.data_as(ctypes.POINTER(_lib.Bin)), len(b),
                 t.ctypes.data_as(ctypes.POINTER(_lib.CellType)), len(t), float(t_max),
                 0.0 if phi is None else float(phi), int(seed))
@@ -233,7 +237,7 @@ class Engine:
         else:
             rc = self.L.pc_simulate(*args, h)
         self._check(rc)
-        return Result(*_lib.histograms_to_numpy(h, 1)[0])
+        return Result(*_lib.histograms_to_numpy(h, own)[0])
 
     def get_option(self, name: str) -> float:
         v = ctypes.c_double()

@@ -209,14 +209,19 @@ class _View:
         self.__array_interface__ = {"data": (address, False), "shape": shape, "typestr": typestr, "version": 3}
 
 
-def histograms_to_numpy(hs, n):
-    """(values, totals, per_type, stats) of each of the n histograms of the ctypes array `hs`,
-    arrays on the library's own memory, which they keep alive (no copy)."""
+def histogram_owners(hs, n):
+    """The owners of the n histograms of the ctypes array `hs`, made before the call that fills them:
+    what a call that fails leaves in them is freed too."""
+    return [_Owner(hs[i]) for i in range(n)]
+
+
+def histograms_to_numpy(hs, owners):
+    """(values, totals, per_type, stats) of each histogram of the ctypes array `hs`, arrays on the
+    library's own memory, which they keep alive (no copy)."""
     out = []
-    for i, (nv, nt, values, totals, per_type) in enumerate(np.frombuffer(hs, HISTOGRAM_DTYPE, n).tolist()):
-        h = hs[i]
-        own = _Owner(h)
-        st = h.stats
+    rows = np.frombuffer(hs, HISTOGRAM_DTYPE, len(owners)).tolist()
+    for own, (nv, nt, values, totals, per_type) in zip(owners, rows):
+        st = own.h.stats
         out.append((np.asarray(_View(own, values, (nv,), "<f8")), np.asarray(_View(own, totals, (nv,), "<u8")),
                     np.asarray(_View(own, per_type, (nv, nt), "<u8")), {k: getattr(st, k) for k in _STATS}))
     return out
