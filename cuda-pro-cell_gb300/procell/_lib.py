@@ -250,10 +250,5 @@ def bins_numpy(bins) -> np.ndarray:
 
 
 def types_numpy(types) -> np.ndarray:
-    if type(types) is list and all(type(t) is tuple and len(t) == 3 for t in types):
-        return np.array(types, TYPE_DTYPE)
-    out = np.empty(len(types), TYPE_DTYPE)
-    for i, (r, m, sd) in enumerate(types):
-        out[i] = (float(r), float(m), float(sd))
-    return out
+    return np.array([(float(r), float(m), float(sd)) for r, m, sd in types], TYPE_DTYPE)
 
