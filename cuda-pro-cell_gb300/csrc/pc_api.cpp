@@ -503,12 +503,34 @@ void parallel_for(uint32_t n, F&& f, unsigned threads = 0) {
 
 // The arrays of result histograms. Large ones come from fresh pages that each cost a fault on
 // first use (a third of the time of reading a 7 MB result), so freed ones are kept for the next
-// results: at most kKept bytes in the process, any thread may allocate or free.
+// results: at most kKept bytes and kBlocks pinned blocks in the process, any thread may allocate
+// or free. With the process's last context what is kept goes back to the system; results may
+// outlive it, and what is freed later is not kept.
 class ResultMemory {
  public:
   static ResultMemory& get() {
     static ResultMemory* r = new ResultMemory();
     return *r;
+  }
+  void attach() {
+    std::lock_guard<std::mutex> lock(m_);
+    ++contexts_;
+  }
+  void detach() {
+    std::lock_guard<std::mutex> lock(m_);
+    if (--contexts_ != 0) return;
+    for (const auto& k : kept_) std::free(k.second);
+    kept_.clear();
+    kept_bytes_ = 0;
+    for (Block& b : blocks_)
+      if (b.refs == 0) drop(b);
+  }
+  // What is kept, and the pinned blocks handed out (bytes).
+  size_t bytes() {
+    std::lock_guard<std::mutex> lock(m_);
+    size_t n = kept_bytes_;
+    for (const Block& b : blocks_) n += b.bytes;
+    return n;
   }
   void* allocate(size_t bytes) {
     if (bytes < kSmall) return std::malloc(std::max<size_t>(1, bytes));
@@ -527,12 +549,14 @@ class ResultMemory {
     return p;
   }
   // Pinned memory for the device to write a result's counts into directly (copying 7 MB out of
-  // a staging buffer takes 0.35 ms): nullptr when none of kBlocks is free or large enough. Its
-  // `refs` arrays are handed out with give_pinned and released one by one.
+  // a staging buffer takes 0.35 ms): nullptr when none of kBlocks is free or large enough. Its two
+  // arrays are handed out with give_pinned and released one by one; one that is taken counts as a
+  // reference too.
   struct Block {
     void* p = nullptr;
     size_t bytes = 0;
     int refs = 0;
+    void* arrays[2] = {nullptr, nullptr};
   };
   static constexpr size_t kPinnedFrom = size_t(1) << 20, kPinnedMost = size_t(64) << 20;
   Block* take_pinned(size_t bytes) {
@@ -548,8 +572,7 @@ class ResultMemory {
       grow = &b;
     }
     if (!grow) return nullptr;
-    if (grow->p) cudaFreeHost(grow->p);
-    *grow = Block();
+    drop(*grow);
     if (pc_cuda_malloc_host(&grow->p, bytes) != cudaSuccess) {
       (void)cudaGetLastError();
       grow->p = nullptr;
@@ -559,23 +582,26 @@ class ResultMemory {
     grow->refs = 1;
     return grow;
   }
-  void give_pinned(Block* b, std::initializer_list<void*> arrays) {
+  void give_pinned(Block* b, void* first, void* second) {
+    std::lock_guard<std::mutex> lock(m_);
+    b->arrays[0] = first;
+    b->arrays[1] = second;
+    b->refs = 2;
+  }
+  void untake_pinned(Block* b) {
     std::lock_guard<std::mutex> lock(m_);
     b->refs = 0;
-    for (void* a : arrays) {
-      pinned_[a] = b;
-      ++b->refs;
-    }
   }
   void release(void* p) {
     if (!p) return;
     std::unique_lock<std::mutex> lock(m_);
-    const auto pin = pinned_.find(p);
-    if (pin != pinned_.end()) {
-      --pin->second->refs;
-      pinned_.erase(pin);
-      return;
-    }
+    for (Block& b : blocks_)
+      for (void*& a : b.arrays)
+        if (a == p) {
+          a = nullptr;
+          if (--b.refs == 0 && contexts_ == 0) drop(b);
+          return;
+        }
     const auto it = out_.find(p);
     if (it == out_.end()) {
       lock.unlock();
@@ -584,7 +610,7 @@ class ResultMemory {
     }
     const size_t size = it->second;
     out_.erase(it);
-    if (kept_bytes_ + size <= kKept) {
+    if (contexts_ != 0 && kept_bytes_ + size <= kKept) {
       try {
         kept_.emplace(size, p);
         kept_bytes_ += size;
@@ -598,6 +624,10 @@ class ResultMemory {
 
  private:
   static constexpr size_t kSmall = size_t(64) << 10, kKept = size_t(64) << 20;
+  static void drop(Block& b) {
+    if (b.p) cudaFreeHost(b.p);
+    b = Block();
+  }
   // An array whose size could not be noted is freed instead of kept.
   void note(void* p, size_t size) {
     try {
@@ -611,7 +641,7 @@ class ResultMemory {
   size_t kept_bytes_ = 0;
   static constexpr int kBlocks = 3;
   Block blocks_[kBlocks];
-  std::map<void*, Block*> pinned_;
+  uint64_t contexts_ = 0;  // live in the process
 };
 template <class T>
 T* result_array(uint64_t n) {
@@ -723,6 +753,7 @@ int pc_create(pc_context** out, int device) {
   size_t fr = 0, tot = 0;
   if ((e = cudaMemGetInfo(&fr, &tot)) != cudaSuccess) return bail(e, "cudaMemGetInfo");
   ctx->free_at_start = fr;
+  ResultMemory::get().attach();
   *out = ctx;
   return PC_OK;
   PC_GUARD_END(nullptr)
@@ -762,6 +793,7 @@ void pc_destroy(pc_context* ctx) {
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   delete ctx;
+  ResultMemory::get().detach();
 }
 
 int pc_set_stream(pc_context* ctx, void* stream) {
@@ -1439,7 +1471,7 @@ int device_result(pc_context* ctx, pc_plan* p, pc_histogram* out) {
   struct Pinned {
     ResultMemory::Block* b;
     ~Pinned() {
-      if (b) ResultMemory::get().give_pinned(b, {});
+      if (b) ResultMemory::get().untake_pinned(b);
     }
   } pinned{ResultMemory::get().take_pinned(back)};
   unsigned long long* const hm = pinned.b ? static_cast<unsigned long long*>(pinned.b->p) : ctx->merge_host;
@@ -1461,7 +1493,7 @@ int device_result(pc_context* ctx, pc_plan* p, pc_histogram* out) {
   if (pinned.b) {
     out->totals = reinterpret_cast<uint64_t*>(hm);
     out->per_type = reinterpret_cast<uint64_t*>(hm + nv);
-    ResultMemory::get().give_pinned(pinned.b, {out->totals, out->per_type});
+    ResultMemory::get().give_pinned(pinned.b, out->totals, out->per_type);
     pinned.b = nullptr;
   } else {
     out->totals = result_array<uint64_t>(nv);
@@ -1627,6 +1659,8 @@ int pc_get_option(pc_context* ctx, const char* name, double* value) {
     *value = (double)g_live_device_allocs.load();
   } else if (n == "level_buffers") {
     *value = (double)ctx->pool.size();
+  } else if (n == "result_memory") {
+    *value = (double)ResultMemory::get().bytes();
   } else {
     return fail(ctx, PC_ERR_INVALID, "unknown option " + n);
   }

@@ -147,7 +147,8 @@ int pc_set_option(pc_context* ctx, const char* name, double value);
 /* Counters for those tests (no counterpart in the reference): "cuda_calls" (CUDA calls the
  * library made for this context so far), "faults_injected", "device_allocations" (device
  * allocations of the library live in this process, all contexts), "level_buffers" (level
- * buffers the context's pool holds). */
+ * buffers the context's pool holds), "result_memory" (bytes of host memory kept for result
+ * arrays in this process, and of the pinned blocks handed out with them). */
 int pc_get_option(pc_context* ctx, const char* name, double* value);
 
 /* phi == 0 selects the reference's automatic threshold: the smallest value with a
@@ -177,6 +178,9 @@ void pc_plan_destroy(pc_plan* plan);
 /* One call: plan, run, result, destroy. */
 int pc_simulate(pc_context* ctx, const pc_bin* bins, uint64_t n_bins, const pc_cell_type* types,
                 uint32_t n_types, double t_max, double phi, uint64_t seed, pc_histogram* out);
+/* Frees a result's arrays, from any thread, before or after its context is destroyed. Freed
+ * arrays of 64 KB and more are kept for the next results: at most 64 MB of pages and three
+ * pinned blocks of up to 64 MB in the process, returned with its last context. */
 void pc_histogram_free(pc_histogram* h);
 
 /* Sharding (one process or GPU per shard): pc_simulate on initial cells [root_begin,

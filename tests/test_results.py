@@ -55,3 +55,52 @@ def test_batches_from_overlapping_threads(built):
     assert not errors
     for a, b in zip(*got):
         assert np.array_equal(a.values, b.values) and np.array_equal(a.per_type, b.per_type)
+
+
+KEPT = r'''
+import gc, sys
+sys.path.insert(0, sys.argv[1])
+import numpy as np
+import test_results as T
+from procell import Engine
+
+def kept():
+    e = Engine(0)
+    n = e.get_option("result_memory")
+    e.close()
+    return n
+
+two = [Engine(0), Engine(0)]
+small = [two[0].simulate(*T.wide_input(s, bins=2000)) for s in range(3)]  # pages, below the pinned threshold
+large = [two[1].simulate(*T.wide_input(s)) for s in range(5)]             # pinned blocks and pages
+want = [r.per_type.copy() for r in large]
+del small
+two[0].close()
+assert two[1].get_option("result_memory") > 0
+two[1].close()
+held = kept()
+assert held > 0, held  # the pinned blocks of the results still held
+for r, w in zip(large, want):
+    assert np.array_equal(r.per_type, w)
+del r, large
+gc.collect()
+assert kept() == 0, kept()
+e = Engine(0)  # and again from nothing
+r = e.simulate(*T.wide_input(3))
+assert np.array_equal(r.per_type, want[3])
+e.close()
+print("kept ok")
+'''
+
+
+def test_kept_memory_goes_back_with_the_last_context(built):
+    """In a process of its own, where no other context is alive."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    pkg = os.path.join(os.path.dirname(here), "cuda-pro-cell_gb300")
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([pkg, os.environ.get("PYTHONPATH", "")]))
+    r = subprocess.run([sys.executable, "-c", KEPT, here], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, (r.stdout[-1000:], r.stderr[-3000:])
+    assert "kept ok" in r.stdout
