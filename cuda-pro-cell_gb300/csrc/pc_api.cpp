@@ -840,7 +840,12 @@ int pc_set_option(pc_context* ctx, const char* name, double value) {
   } else {
     return fail(ctx, PC_ERR_INVALID, "unknown option " + n);
   }
-  if (n == "memory_budget_bytes" || n == "grid_blocks") free_pool(ctx);
+  if (n == "memory_budget_bytes" || n == "grid_blocks") {
+    free_pool(ctx);
+    pc_cuda_free(ctx->walk_dev);  // every run is over; a captured one is captured again
+    ctx->walk_dev = nullptr;
+    ctx->walk_bytes = 0;
+  }
   return PC_OK;
   PC_GUARD_END(ctx)
 }

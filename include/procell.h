@@ -109,8 +109,11 @@ const char* pc_version(void);
 int pc_set_stream(pc_context* ctx, void* stream);
 
 /* Tuning knobs (results never depend on them):
- *   "memory_budget_bytes" device bytes the level buffers may use (default: half of the
- *                         free memory at first use)
+ *   "memory_budget_bytes" device bytes the level buffers or the tree walk's scratch may use
+ *                         (default: half of the free memory at first use). The scratch is
+ *                         sized by the deepest phi cap, not by the run: 124 MB at 14
+ *                         generations, 187 MB at 31, once per context; with less, the sweeps
+ *                         run instead. Setting it gives both kinds back.
  *   "max_slice_cells"     cap on cells per division-sweep launch (default: from budget)
  *   "max_root_chunk"      cap on roots per root-sweep launch (default: from budget)
  *   "grid_blocks"         blocks per launch (default: resident blocks x SMs)
@@ -119,6 +122,8 @@ int pc_set_stream(pc_context* ctx, void* stream);
  *                         max_root_chunk set, a run whose phi caps are at most 31 is one
  *                         tree walk instead (one cooperative launch, no level buffers;
  *                         stats count its rounds as sweeps); the sweeps serve the rest.
+ *                         A tree walk takes every SM for its duration, also for a few
+ *                         cells: runs of two contexts follow one another on the device.
  *   "driver"              0: one kernel launch per sweep (default); 1: one persistent
  *                         cooperative launch per run
  *   "graph"               1: the persistent driver captures its run in a CUDA graph once

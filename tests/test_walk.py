@@ -191,3 +191,30 @@ def test_a_walk_without_scratch_goes_to_the_level_sweeps(oracle_lib):
             eng.close()
         n += 1
     assert n > 5 and by_sweeps == 1
+
+
+@pytest.mark.gpu
+def test_the_memory_budget_bounds_the_scratch(oracle_lib):
+    """Setting the budget gives the walk's scratch back; below its size the level sweeps run, and a
+    run captured in a graph before is captured again on the new scratch."""
+    import procell.configs as cfg
+    from procell import Engine
+    w = cfg.small()
+    o = oracle_lib.simulate(w.bins, w.types, w.t_max, w.phi, seed=w.seed, nthreads=0)
+    eng = Engine(0)
+    try:
+        eng.set_option("driver", 1)
+        eng.set_option("graph", 1)
+        p = eng.plan(w.bins, w.types, w.t_max, w.phi, w.seed)
+        p.run()
+        for budget in (1 << 30, 32 << 20, 1 << 30):
+            before = eng.get_option("device_allocations")
+            eng.set_option("memory_budget_bytes", budget)
+            assert eng.get_option("device_allocations") < before
+            for _ in range(2):
+                p.run()
+                assert np.array_equal(p.result().per_type, o.per_type)
+            assert (eng.get_option("level_buffers") > 0) == (budget == 32 << 20)
+        p.close()
+    finally:
+        eng.close()
