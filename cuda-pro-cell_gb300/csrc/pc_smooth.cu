@@ -62,6 +62,17 @@ constexpr int kBlocksDrawn = 6;
 constexpr int kBlocksKept = 7;
 constexpr int kBlocksKeptJacobian = 6;
 constexpr int kBlocksKeptAdjoint = 6;
+// The adjoint's pairs keep three waiting floats per generation row and thread in shared memory, so
+// their resident blocks fall with the plan's deepest bin: 6 up to 15 rows, 4 up to 24, 3 up to 32,
+// 1 at 64. Deeper plans walk one lineage at a time, 8 blocks per SM, which is never slower than pairs
+// were there: 255 bins of ordinary brightness and one bright one, 256 candidates, adjoint with
+// pairs and without: 16 rows 0.313 and 0.333 ms, 23 0.350 and 0.333, 25 0.418 and 0.334, 33 0.557
+// and 0.334, 64 1.008 and 0.503; 5 candidates 0.104 and 0.123, 0.112 and 0.120, 0.125 and 0.120,
+// 0.134 and 0.120, 0.257 and 0.204. (Few blocks of long walks gain from pairs at any depth, 64 deep
+// bins 0.13 and 0.23 ms, but how long the walks are depends on the candidates, and one candidate's
+// result is not to depend on the others.)
+constexpr int kBlocksKeptAdjointSingle = 8;
+constexpr uint32_t kPairRowsAdjoint = 24;
 
 __device__ __forceinline__ double f32_to_f64_bits(float z) {
   const uint32_t f = __float_as_uint(z);
@@ -754,8 +765,11 @@ __global__ void __launch_bounds__(kThreads, Kept ? kBlocksKeptJacobian : kBlocks
 // Forward (e_raw[c][k][b][g] = ratio_k / paths * sum 2^g w_g over the bin's lineages) and
 // adjoint (part[c][b][3k + q] = d(sum_g A_g E_g)/d(ratio_k, mean_k, sd_k)) of one type: block
 // (bin, group of 32 candidates, type k). Every block draws its bin's lineages itself.
-template <bool Backward, bool Kept>
-__global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoint : kBlocksKept) : kBlocksDrawn) k_smooth(const SmoothArgs A, const double* __restrict__ params,
+template <bool Backward, bool Kept, bool Pairs>
+__global__ void __launch_bounds__(kThreads, !Kept      ? kBlocksDrawn
+                                            : !Backward ? kBlocksKept
+                                            : Pairs     ? kBlocksKeptAdjoint
+                                                        : kBlocksKeptAdjointSingle) k_smooth(const SmoothArgs A, const double* __restrict__ params,
                                                      uint32_t ncand, const double* __restrict__ grad_expected,
                                                      uint32_t nvalues, const int32_t* __restrict__ vidx,
                                                      double* __restrict__ out) {
@@ -774,7 +788,7 @@ __global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoin
   const uint32_t KQ = A.ntypes * 3u;
   const uint32_t arows = Backward ? 6u : 2u * A.rows;
   float* zbuf = facc + (size_t)arows * kThreads + (size_t)warp * A.rows * 32u;
-  // adjoint: 2^g dL/dE_g [rows][32 lanes], then the waiting terms [3 rows][kThreads]
+  // adjoint: 2^g dL/dE_g [rows][32 lanes], then the waiting terms [3 rows][kThreads] of pairs
   float* const Ag2 = facc + (size_t)(arows + A.rows) * kThreads;
   float* const later = Ag2 + 32u * A.rows + threadIdx.x;
   if constexpr (!Kept)
@@ -794,11 +808,11 @@ __global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoin
         if (v >= 0) a = ldexp(grad_expected[(uint64_t)cc * nvalues + v], (int)g);
       }
       Ag2[i] = (float)a;
-      finite = finite && isfinite((float)a);
+      if constexpr (Pairs) finite = finite && isfinite((float)a);
     }
     // A gradient that is not finite (FP32) is left out where a weight is 0, which walk() looks
     // for and a pair does not: the whole block walks alone.
-    finite = __syncthreads_and(finite) != 0;
+    if constexpr (Pairs) finite = __syncthreads_and(finite) != 0;
   }
   const double* my_prm = params + (uint64_t)(live ? c : 0u) * KQ + 3u * k;
   const double mu = live ? my_prm[1] : 0.0, sd = live ? my_prm[2] : 0.0;
@@ -814,7 +828,7 @@ __global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoin
   RemGrid rg;
   const bool grid = opaque(grid_shared(rg, mu, sd, A.t_max, steps, A.h, reinterpret_cast<float*>(u_age)));
   const RemFp64 rd{mu, sd, A.t_max, 0.0};
-  const bool pairs = opaque(grid && walks && finite && !quiescent && !fixed_tau);
+  const bool pairs = Pairs && opaque(grid && walks && finite && !quiescent && !fixed_tau);
   const RemGrid2 rg2(rg, rg);
   const float stop = stop_level(steps);  // once per block: the walks' stopping threshold
   // lineage i of the bin: initial cell r0 + i / paths, replica i % paths
@@ -829,15 +843,16 @@ __global__ void __launch_bounds__(kThreads, Kept ? (Backward ? kBlocksKeptAdjoin
     if (live) {
       float f_r = 0.0f, f_mu = 0.0f, f_sig = 0.0f;  // adjoint terms of these (up to) 32 lineages
       const uint32_t n2 = pairs ? n & ~1u : 0u;  // lineages taken two at a time
-      for (uint32_t ii = 0; ii < n2; ii += 2u) {
-        const uint32_t li = warp * 32u + ii;
-        const f2 u = *reinterpret_cast<const f2*>(u_one + li), u_lo = *reinterpret_cast<const f2*>(u_one_lo + li);
-        if constexpr (Backward)
-          walk_adjoint(reinterpret_cast<const f2*>(zbuf + ii), u, u_lo, inv_h, steps, stop, rg2, later, my_ag, f_r, f_mu,
-                       f_sig);
-        else
-          walk_lineages<false>(reinterpret_cast<const f2*>(zbuf + ii), u, u_lo, inv_h, steps, stop, rg2, fmy);
-      }
+      if constexpr (Pairs)
+        for (uint32_t ii = 0; ii < n2; ii += 2u) {
+          const uint32_t li = warp * 32u + ii;
+          const f2 u = *reinterpret_cast<const f2*>(u_one + li), u_lo = *reinterpret_cast<const f2*>(u_one_lo + li);
+          if constexpr (Backward)
+            walk_adjoint(reinterpret_cast<const f2*>(zbuf + ii), u, u_lo, inv_h, steps, stop, rg2, later, my_ag, f_r,
+                         f_mu, f_sig);
+          else
+            walk_lineages<false>(reinterpret_cast<const f2*>(zbuf + ii), u, u_lo, inv_h, steps, stop, rg2, fmy);
+        }
       for (uint32_t ii = n2; ii < n; ++ii) {
         if (quiescent) {
           // quiescent type: a leaf at generation 0 (cell.cu:69-75)
@@ -1113,30 +1128,32 @@ __global__ void k_smooth_grad_sum(const double* __restrict__ part, uint32_t ncan
 
 // accumulator pairs (2 floats per output row and thread) + the lineage draws (kThreads
 // floats per generation row) + the adjoint's gradients and waiting terms
-int smem_bytes(bool backward, uint32_t rows) {
-  return (int)((backward ? (6u + 4u * rows) * kThreads + 32u * rows : 3u * rows * kThreads) * sizeof(float));
+int smem_bytes(bool backward, bool pairs, uint32_t rows) {
+  return (int)((backward ? (6u + (pairs ? 4u : 1u) * rows) * kThreads + 32u * rows : 3u * rows * kThreads) * sizeof(float));
 }
 
-template <bool Backward, bool Kept>
+template <bool Backward, bool Kept, bool Pairs>
 int launch_smooth_k(const SmoothArgs& A, const double* params, uint32_t ncand, const double* grad_expected,
                     uint32_t nvalues, const int32_t* vidx, double* out, cudaStream_t st) {
-  const int smem = smem_bytes(Backward, A.rows);
+  const int smem = smem_bytes(Backward, Pairs, A.rows);
   // static shared memory plus `smem` may exceed the default 48 KB: always opt in
   const cudaError_t e =
-      cudaFuncSetAttribute(k_smooth<Backward, Kept>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      cudaFuncSetAttribute(k_smooth<Backward, Kept, Pairs>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
   const int eo = launch_order(A, params, ncand, st);
   if (eo != 0) return eo;
   const dim3 grid(A.nbins, (ncand + 31u) / 32u, A.ntypes);
-  k_smooth<Backward, Kept><<<grid, kThreads, smem, st>>>(A, params, ncand, grad_expected, nvalues, vidx, out);
+  k_smooth<Backward, Kept, Pairs><<<grid, kThreads, smem, st>>>(A, params, ncand, grad_expected, nvalues, vidx, out);
   return (int)cudaGetLastError();
 }
 
 template <bool Backward>
 int launch_smooth_t(const SmoothArgs& A, const double* params, uint32_t ncand, const double* grad_expected,
                     uint32_t nvalues, const int32_t* vidx, double* out, cudaStream_t st) {
-  return A.lin_z ? launch_smooth_k<Backward, true>(A, params, ncand, grad_expected, nvalues, vidx, out, st)
-                 : launch_smooth_k<Backward, false>(A, params, ncand, grad_expected, nvalues, vidx, out, st);
+  auto* launch = A.lin_z ? launch_smooth_k<Backward, true, true> : launch_smooth_k<Backward, false, true>;
+  if constexpr (Backward)
+    if (A.rows > kPairRowsAdjoint) launch = A.lin_z ? launch_smooth_k<true, true, false> : launch_smooth_k<true, false, false>;
+  return launch(A, params, ncand, grad_expected, nvalues, vidx, out, st);
 }
 
 // The Jacobian kernel of a plan that keeps its lineage draws or not.

@@ -139,3 +139,35 @@ def test_gradient_that_is_not_finite_where_no_cell_is(engine, bad):
         assert np.all(np.isfinite(got[1]))
         assert np.all(np.abs(got[1] - got[0]) <= tol)
     assert hit > 0
+
+
+@pytest.mark.parametrize("predraw", [1, 0])
+@pytest.mark.parametrize("extra", [23, 24, 25, 63])  # the plan's rows are one more: pairs up to 24 rows
+def test_adjoint_of_plans_with_a_deep_bin(engine, predraw, extra):
+    """The same bins in a plan by themselves (pairs) and with a brighter bin behind them, whose depth
+    decides how the whole plan is walked and whose own gradient is 0: the same lineages, so the same
+    adjoint up to rounding. Tolerance as in test_pairs_against_single_walks."""
+    import torch
+    from procell.smooth import Smooth
+    bins = [(900.0, 35), (77.0, 3), (3.0, 4), (150.0, 64)]
+    P = torch.tensor([[[0.5, 22.0, 4.0], [0.5, 35.0, 14.0]], [[0.3, 60.0, 3.0], [0.7, 18.0, 9.0]]], device="cuda",
+                     dtype=torch.float64)
+    rng = np.random.default_rng(extra)
+    engine.set_option("smooth_predraw", predraw)
+    try:
+        sm = Smooth(engine, bins, n_types=2, t_max=140.0, phi=1.0, h=0.5, paths=1, seed=31)
+        values, g = list(sm.values), rng.normal(size=(2, sm.n_values))
+        J = sm.jacobian(P)[1].cpu().numpy()
+        alone = sm.backward(P, torch.tensor(g, device="cuda")).cpu().numpy()
+        sm.sync()
+        sm.close()
+        sm = Smooth(engine, bins + [(1.5 * 2.0 ** extra, 2)], n_types=2, t_max=140.0, phi=1.0, h=0.5, paths=1, seed=31)
+        grad = np.zeros((2, sm.n_values))
+        grad[:, [list(sm.values).index(v) for v in values]] = g
+        both = sm.backward(P, torch.tensor(grad, device="cuda")).cpu().numpy()
+        sm.sync()
+        sm.close()
+    finally:
+        engine.set_option("smooth_predraw", 1)
+    terms = np.einsum("cv,cvkq->ckq", np.abs(g), np.abs(J))
+    assert np.all(np.abs(both - alone) <= (64 * 64 + 2) * 2.0 ** -24 * terms + 1e-10)
