@@ -177,11 +177,6 @@ __device__ __forceinline__ void stack_put(WalkWarp<Batched>& W, uint32_t i, uint
   W.stack_m[i] = make_uint2(e.z, e.w);
 }
 
-// Sum over the warp of 32-bit values, as 64 bits.
-__device__ __forceinline__ unsigned long long warp_sum32(uint32_t v) {
-  return __reduce_add_sync(kFull, v & 0xFFFFu) + ((unsigned long long)__reduce_add_sync(kFull, v >> 16) << 16);
-}
-
 // The warp's global region of a round: cells spilled, then handed over.
 __device__ __forceinline__ uint4* walk_region(const WalkArgs& w, uint32_t round) {
   const uint32_t wid = blockIdx.x * kWalkWarps + (threadIdx.x >> 5);
@@ -189,39 +184,52 @@ __device__ __forceinline__ uint4* walk_region(const WalkArgs& w, uint32_t round)
 }
 
 // The window into the global table: leaves(g) = 2 D(g - 1) - D(g) - (g == cap ? V : 0), in
-// wrapping arithmetic (a cell handed over is counted by another warp than its parent).
+// wrapping arithmetic (a cell handed over is counted by another warp than its parent). Lanes c
+// and 16 + c take column c's even and odd generations. At most 2^30 cells are counted between two
+// flushes, so 32 bits hold their sums.
+// A window is flushed whenever the next initial cells bring a 17th class: every 20 to 60 cells where
+// a bin has many types or few cells. One column after another, lanes as generations, took 45
+// instructions each. 1.6e7 cells of 24 types, 1.25 divisions each: 2.23 -> 1.75 ms; 4e6 cells in
+// bins of 8, 8 types 0.72 -> 0.58; 512 instances of 4096 cells and 24 types 0.63 -> 0.54.
 template <bool Batched>
 __device__ __noinline__ void walk_flush(uint32_t ncols) {
   const RunArgs& a = walk_shared<Batched>().w.a;
   WalkWarp<Batched>& W = walk_warp<Batched>();
-  const uint32_t lane = threadIdx.x & 31u;
-  unsigned long long divisions = 0, vanished = 0;
-  uint32_t gens = 0;  // bit g: a cell of generation g divided
+  const uint32_t lane = threadIdx.x & 31u, c = lane & 15u;
   __syncwarp();
-  for (uint32_t c = 0; c < ncols; ++c) {
-    const uint2 x = W.aux[c];
-    const uint32_t cap = (x.y >> 16) & 0xFFu;
-    uint32_t* col = W.window + c * kColWords;
-    const uint32_t dl = lane < cap ? col[cap - lane] : 0u;  // D(lane)
-    const uint32_t v = col[0];
-    __syncwarp();
-    col[lane] = 0u;
-    const uint32_t dm = __shfl_up_sync(kFull, dl, 1);
-    unsigned long long leaves = 0ull;
-    if (lane != 0u) {
-      leaves = 2ull * dm - dl;
-      if (lane == cap) leaves -= v;
+  const uint2 x = W.aux[c];
+  const int cap = c < ncols ? (int)((x.y >> 16) & 0xFFu) : -1;
+  const uint32_t last = (uint32_t)__reduce_max_sync(kFull, cap);
+  uint32_t* const word = W.window + c * kColWords + cap;  // D(0); D(g) g words before it, V at g = cap
+  uint32_t divisions = 0, vanished = 0, deepest = 0, before = 0;
+  if (ncols != 0u)
+    for (uint32_t g = lane >> 4; g <= last + (lane >> 4); g += 2u) {
+      uint32_t d = 0, v = 0;
+      if ((int)g <= cap) {
+        d = word[-(int)g];
+        word[-(int)g] = 0u;
+        if ((int)g == cap) {
+          v = d;
+          d = 0;
+        }
+      }
+      // D(g - 1): the odd lane's of the step before, the even lane's of this one
+      const uint32_t above = __shfl_xor_sync(kFull, lane < 16u ? d : before, 16);
+      before = d;
+      const unsigned long long leaves = 2ull * above - d - v;
+      if (g != 0u && leaves != 0ull && in_bounds(g < a.hist_gens && x.x < a.nclass, a.error))
+        atomicAdd(a.hist + (uint64_t)g * a.nclass + x.x, leaves);
+      divisions += d;
+      vanished += v;
+      if (d != 0u) deepest = g + 1u;
     }
-    if (leaves != 0ull && in_bounds(lane < a.hist_gens && x.x < a.nclass, a.error))
-      atomicAdd(a.hist + (uint64_t)lane * a.nclass + x.x, leaves);
-    divisions += warp_sum32(dl);
-    vanished += v;
-    gens |= __ballot_sync(kFull, dl != 0u);
-  }
+  divisions = __reduce_add_sync(kFull, divisions);
+  vanished = __reduce_add_sync(kFull, vanished);
+  deepest = __reduce_max_sync(kFull, deepest);
   if (lane == 0u) {
     W.divisions += divisions;
     W.vanished += vanished;
-    W.max_gen = max(W.max_gen, 32u - (uint32_t)__clz((int)gens));
+    W.max_gen = max(W.max_gen, deepest);
   }
   __syncwarp();
 }
