@@ -2066,9 +2066,10 @@ int run_walk(pc_context* ctx, pc_plan* p, const RunArgs& a) {
   w.root_lo = p->root_begin;
   w.root_hi = p->root_end;
   w.batch = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(4, (nroots + warps - 1) / warps));
-  // initial cells of a range share bins, hence window columns; small enough that the ranges
-  // still deal the work out evenly
-  w.chunk = (uint32_t)std::min<uint64_t>(256, std::max<uint64_t>(w.batch, nroots / (warps * 4) / 32 * 32));
+  // initial cells of a range share bins, hence window columns, and the search for its first bin;
+  // small enough that the ranges still deal the work out evenly (1.6e7 cells in 5e5 bins, 4 types,
+  // 1.25 divisions each: 256 cells 0.94 ms, 512 0.88, 1024 0.89; 24 types 1.80, 1.73 and 1.91)
+  w.chunk = (uint32_t)std::min<uint64_t>(512, std::max<uint64_t>(w.batch, nroots / (warps * 4) / 32 * 32));
   w.timeout_ns = 60000000000ull;
   // a stack holds at most about 32 cells per generation; a region that overflows all the same
   // sets an error bit and the run goes to the level sweeps
