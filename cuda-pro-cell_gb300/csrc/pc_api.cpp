@@ -700,6 +700,9 @@ bool host_walk_type(TypeDev& t, double mean, double sd, double t_max) {
   if (!(t_max == 0.0 || t_max >= lo) || !(t_max <= hi)) return false;
   if (t.mode == kModeQuiescent) return true;
   const bool zero = t.mode == kModeZeroMean;
+  // every cell of such a type has a time left of exactly 0, inside any band: each would replay its
+  // lineage (4000 cells in 64 bins, 1.14 ms; the level sweeps 0.46)
+  if (zero && t_max == 0.0) return false;
   if (!zero && !(mean >= lo && mean <= hi && std::fabs(sd) <= hi)) return false;
   t.w_mean = zero ? 0.0f : (float)mean;
   t.w_sd = zero ? 0.0f : (float)sd;

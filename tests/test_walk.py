@@ -218,3 +218,14 @@ def test_the_memory_budget_bounds_the_scratch(oracle_lib):
         p.close()
     finally:
         eng.close()
+
+
+@pytest.mark.gpu
+def test_cells_that_are_all_due_at_once_go_to_the_level_sweeps(engine, oracle_lib):
+    """Zero-mean types at t_max = 0: a time left of 0 is inside every band, so the walk would settle
+    every cell by replaying its lineage."""
+    bins, types, t_max = CASES["zero_mean_at_zero"]
+    g = engine.simulate(bins, types, t_max, 1.0, 4242)
+    o = oracle_lib.simulate(bins, types, t_max, 1.0, seed=4242, nthreads=0)
+    assert np.array_equal(g.per_type, o.per_type) and g.stats["divisions"] == o.stats["divisions"]
+    assert g.stats["kernel_launches"] > 1  # a walk is one launch
