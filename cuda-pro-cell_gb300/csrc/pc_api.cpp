@@ -1331,22 +1331,26 @@ int instance_result(const pc_plan* p, const InstanceHost& I, const unsigned long
     std::memset(out->per_type, 0, nv * nt * sizeof(uint64_t));
   }
   uint64_t leaves = 0;
-  for (uint32_t g = 0; g < I.hist_gens; ++g)
-    for (uint32_t b = 0; b < nb; ++b) {
+  const uint32_t* const to_file = I.sorted_to_file.data();
+  for (uint32_t g = 0; g < I.hist_gens; ++g) {
+    const unsigned long long* row = h + g * p->nclass + I.class_begin;
+    for (uint32_t b = 0; b < nb; ++b, row += nt) {
       const int64_t vi = I.vidx[(uint64_t)b * I.vidx_stride + g];
+      uint64_t sum = 0;
       for (uint32_t k = 0; k < nt; ++k) {
-        const uint64_t c = h[g * p->nclass + I.class_begin + (uint64_t)b * nt + k];
-        if (!c) continue;
+        if (!row[k]) continue;
         if (vi < 0) {
           pc_histogram_free(out);
           *msg = "internal: leaf counted outside the output value set";
           return PC_ERR_CUDA;
         }
-        out->totals[vi] += c;
-        out->per_type[(uint64_t)vi * nt + I.sorted_to_file[k]] += c;
-        leaves += c;
+        out->per_type[(uint64_t)vi * nt + to_file[k]] += row[k];
+        sum += row[k];
       }
+      if (sum != 0) out->totals[vi] += sum;
+      leaves += sum;
     }
+  }
   out->stats.leaves = leaves;
   return PC_OK;
 }
