@@ -2078,9 +2078,7 @@ int run_walk(pc_context* ctx, pc_plan* p, const RunArgs& a) {
   // 1.25 divisions each: 256 cells 0.94 ms, 512 0.88, 1024 0.89; 24 types 1.80, 1.73 and 1.91)
   w.chunk = (uint32_t)std::min<uint64_t>(512, std::max<uint64_t>(w.batch, nroots / (warps * 4) / 32 * 32));
   w.timeout_ns = 60000000000ull;
-  // a stack holds at most about 32 cells per generation; a region that overflows all the same
-  // sets an error bit and the run goes to the level sweeps
-  w.region_stride = 32ull * (p->gmax + 2u) + 512u;
+  w.region_stride = walk_region_cells(p->gmax);
   const size_t per_warp = 2 * (w.region_stride * sizeof(uint4) + 2 * kWalkCols * sizeof(uint4) + sizeof(uint4) +
                                sizeof(ulonglong2));
   const size_t need = warps * per_warp;

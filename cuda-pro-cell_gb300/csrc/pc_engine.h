@@ -199,6 +199,7 @@ struct WalkArgs {
 
 int walk_occupancy(bool batched, int* blocks_per_sm);
 uint32_t walk_warps_per_block();
+uint32_t walk_region_cells(uint32_t gmax);  // cells of a warp's global region
 int launch_walk(const WalkArgs& w, int blocks, void* stream);  // cooperative launch
 
 // One compiled configuration of the sweeps (the autotuner's search space): threads per

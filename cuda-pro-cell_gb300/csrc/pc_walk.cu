@@ -15,6 +15,18 @@ int walk_occupancy(bool batched, int* blocks_per_sm) {
 
 uint32_t walk_warps_per_block() { return kWalkWarps; }
 
+// A stack holds at most about 32 cells per generation; a region that overflows all the same (parked
+// cells may come back to a deep stack) sets an error bit and the run goes to the level sweeps, which
+// a build with a small region makes happen for a test.
+uint32_t walk_region_cells(uint32_t gmax) {
+#ifdef PC_WALK_REGION_CELLS
+  (void)gmax;
+  return PC_WALK_REGION_CELLS;
+#else
+  return 32u * (gmax + 2u) + 512u;
+#endif
+}
+
 int launch_walk(const WalkArgs& w, int blocks, void* stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)blocks);

@@ -229,3 +229,32 @@ def test_cells_that_are_all_due_at_once_go_to_the_level_sweeps(engine, oracle_li
     o = oracle_lib.simulate(bins, types, t_max, 1.0, seed=4242, nthreads=0)
     assert np.array_equal(g.per_type, o.per_type) and g.stats["divisions"] == o.stats["divisions"]
     assert g.stats["kernel_launches"] > 1  # a walk is one launch
+
+
+# Timers close to exponential ones (a normal of mean far below its spread, cut at 0): about 5e5
+# divisions whose deepest lineages reach the cap of 31, where a node takes all 32 bits.
+AT_CAP_31 = ([(2.0 ** 31.5, 2), (2.0 ** 31.2, 1)], [(1.0, 0.25, 10.0)], 120.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("driver,graph", [(0, 0), (1, 1)])
+def test_lineages_that_reach_the_cap_of_31(engine, oracle_lib, driver, graph):
+    o = oracle_lib.simulate(*AT_CAP_31, 1.0, seed=4242, nthreads=0)
+    assert o.stats["max_gen"] == 31 and o.stats["vanished"] > 1000
+    engine.set_option("driver", driver)
+    engine.set_option("graph", graph)
+    try:
+        g = engine.simulate(*AT_CAP_31, 1.0, 4242)
+        b = engine.batch([(*CASES["warp_edges"], 1.0, 7), (*AT_CAP_31, 1.0, 4242), (*CASES["cap_31"], 1.0, 9)])
+        b.run()
+        in_batch, beside = b.result(1), b.result(2)
+        b.close()
+    finally:
+        engine.set_option("driver", 0)
+        engine.set_option("graph", 0)
+    assert np.array_equal(g.per_type, o.per_type) and np.array_equal(in_batch.per_type, o.per_type)
+    for k in ("divisions", "vanished", "uncounted", "leaves"):
+        assert g.stats[k] == o.stats[k], k
+    assert g.stats["max_generation"] == 31
+    o2 = oracle_lib.simulate(*CASES["cap_31"], 1.0, seed=9, nthreads=0)
+    assert np.array_equal(beside.per_type, o2.per_type)
