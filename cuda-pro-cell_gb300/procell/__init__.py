@@ -99,8 +99,8 @@ def instance_array(instances):
             bins, types, t_max, phi, seed = inst
         b, t = _lib.bins_numpy(bins), _lib.types_numpy(types)
         keep += [b, t]
-        rows.append((b.__array_interface__["data"][0], len(b), t.__array_interface__["data"][0], len(t), 0, float(t_max),
-                     0.0 if phi is None else float(phi), int(seed) & 0xFFFFFFFFFFFFFFFF))
+        rows.append((b.ctypes.data, len(b), t.ctypes.data, len(t), 0, float(t_max), 0.0 if phi is None else float(phi),
+                     int(seed) & 0xFFFFFFFFFFFFFFFF))
     arr = (_lib.Instance * max(1, len(instances)))()
     if rows:
         np.frombuffer(arr, _lib.INSTANCE_DTYPE, len(rows))[:] = rows
