@@ -126,10 +126,11 @@ __device__ __forceinline__ void kahan_add(float* p, float x) {
 
 // sigmoid(x) and 1 - sigmoid(x) from e = exp(-|x|) and one reciprocal: 1 / (1 + e) is the
 // larger of the two and e / (1 + e) the smaller (for x >= 0, sigmoid(x) is the larger), so
-// both keep their relative accuracy however far x is from 0. With the fast exp and
-// reciprocal intrinsics (relative errors near 2^-22) each factor of a weight is good to a few
-// 1e-7, and a weight of up to ~60 factors to about 1e-5 at worst (checked against the FP64
-// CPU restatement to 2e-5 and against central differences to 1e-3).
+// both keep their relative accuracy however far x is from 0. With the fast exp and reciprocal
+// intrinsics the smaller one is good to about 2^-21.5 + |x| 2^-23.7. A walk ends once its product is
+// below e^-40 2^-steps, so the |x| of the smaller factors in it add up to at most 84 and their
+// second terms to 7e-6; a weight of up to ~60 factors is good to about 1e-5 (checked against the
+// FP64 CPU restatement to 2e-5 and against central differences to 1e-3).
 __device__ __forceinline__ void sig_pair(float x, float& s, float& one_m_s) {
   const float e = __expf(-fabsf(x));
   const float q = __fdividef(1.0f, 1.0f + e);
@@ -541,12 +542,13 @@ struct RemGrid2 {
 };
 
 // exp(-|x|) = 2^(-|x| log2 e) and 1 / y by the ISA's approximate instructions in their flushing
-// form (relative errors near 2^-22 for |x| up to a few tens, and 2^-23). The intrinsics __expf and
-// __fdividef also serve subnormal results and any y, which costs instructions in every step and
-// which no pair needs: y is between 1 and 2, and a factor below 2^-126 takes its product below
-// the stopping level, which ends the walk (a bin has at most 64 steps, see stop_level). 256
-// candidates: forward 0.794 -> 0.691, adjoint 0.979 -> 0.862, Jacobian 0.910 -> 0.810 ms (with a
-// walk below that level left to add its last weights, instead of set to 0 in each step).
+// form: relative errors of about 2^-22 + |x| 2^-23.7 (the second term is the rounded argument's,
+// and the intrinsic's as well) and 2^-23. The intrinsics __expf and __fdividef also serve subnormal
+// results and any y, which costs instructions in every step and which no pair needs: y is between 1
+// and 2, and a factor below 2^-126 takes its product below the stopping level, which ends the walk
+// (a bin has at most 64 steps, see stop_level). 256 candidates: forward 0.794 -> 0.691, adjoint
+// 0.979 -> 0.862, Jacobian 0.910 -> 0.810 ms (with a walk below that level left to add its last
+// weights, instead of set to 0 in each step).
 __device__ __forceinline__ float exp_neg(float x) {
   float e;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__fmul_rn(-fabsf(x), 1.4426950408889634f)));

@@ -54,11 +54,14 @@ constexpr int kWalkWarps = kWalkThreads / 32;
 constexpr int kWalkBlocksPerSm = 1;
 constexpr uint32_t kCols = kWalkCols;   // histogram classes in a warp's window
 // Shared-memory stack entries of a warp, parked ones included, and the cells a full step may start
-// with: it pops 32 and adds at most 128, with up to 31 parked before it. A batched run refills its
-// stacks far more often than it overflows them, and its lookups and the local memory of the code
-// around the steps gain more from 32 KB more of L1 than its steps from 80 more cells: 25.6e6
-// initial cells and 1.29e8 divisions 1.86 ms with 400, 1.68 with 320, a plain run of 2.27e9
-// divisions 13.05 and 13.27 ms.
+// with: it pops 32 and adds at most 128, with up to 31 parked before it. 80 cells fewer leave 32 KB
+// more of L1 to the lookups of initial cells and the local memory of the code around the steps, 80
+// more save spills where trees are deep; which is worth more depends on the run, not on its form.
+// 320 and 400 cells, ms: batches of 256 x 1e5 cells (4 divisions each) 1.34 and 1.53, 10 x 1e5 (12)
+// 0.168 and 0.171, 4 x 25000 (270) 0.344 and 0.364, 256 x 1e4 (230) 4.24 and 4.21, 16 x 6.4e5 (210)
+// 13.63 and 13.49; plain runs of 1e7 cells (4) 0.536 and 0.562, 1e6 (13) 0.158 and 0.167, 1e5 (240)
+// 0.302 and 0.322, 1e7 (240) 14.26 and 14.00. Each kernel has the one that its largest loads want:
+// a batch is most often many shallow runs, the longest plain runs are deep.
 template <bool Batched>
 constexpr uint32_t kStackCap = Batched ? 320 : 400;
 template <bool Batched>
