@@ -475,12 +475,21 @@ __device__ __forceinline__ void walk_roots(const WalkSmem<Batched>& S, WalkWarp<
   const u32x4 Q = philox(u32x4{0u, 0u, root, kPurposeRoot}, k0, k1);
   // u < cumulative ratio on the 53-bit integers
   const unsigned long long m = ((unsigned long long)Q.x << 21) | (Q.y >> 11);
-  uint32_t ty = fallback;
-  for (uint32_t i = 0; i < ntypes; ++i)
-    if (m < __ldg(&walk_type<Batched>(a, type_begin + i).w_cum)) {
-      ty = i;
-      break;
-    }
+  // (the first type whose threshold is above m: thresholds need not ascend). Four at a time: a
+  // batch's types rarely stay in L1, and 64 loads one after another set its time (4.2e6 cells of 64
+  // instances with 64 types 1.35 -> 0.94 ms, the level sweeps 1.15; 1.6e7 plain cells 3.29 -> 2.76).
+  auto threshold = [&](uint32_t i) { return __ldg(&walk_type<Batched>(a, type_begin + i).w_cum); };
+  uint32_t ty = fallback, i = 0;
+  bool chosen = false;
+  for (; !chosen && i + 4u <= ntypes; i += 4u) {
+    const unsigned long long b0 = threshold(i), b1 = threshold(i + 1u), b2 = threshold(i + 2u), b3 = threshold(i + 3u);
+    chosen = m < b0 || m < b1 || m < b2 || m < b3;
+    if (chosen) ty = i + (m < b0 ? 0u : m < b1 ? 1u : m < b2 ? 2u : 3u);
+  }
+  for (; !chosen && i < ntypes; ++i) {
+    chosen = m < threshold(i);
+    if (chosen) ty = i;
+  }
   const uint32_t info = __ldg(a.bin_info + bin), cap = info & 0xFFu;
   const uint32_t cls = Batched ? __ldg(a.bin_class + bin) + ty : bin * a.ntypes + ty;
   const TypeDev& T = walk_type<Batched>(a, type_begin + ty);

@@ -258,3 +258,19 @@ def test_lineages_that_reach_the_cap_of_31(engine, oracle_lib, driver, graph):
     assert g.stats["max_generation"] == 31
     o2 = oracle_lib.simulate(*CASES["cap_31"], 1.0, seed=9, nthreads=0)
     assert np.array_equal(beside.per_type, o2.per_type)
+
+
+@pytest.mark.gpu
+def test_type_choice_of_every_count(engine, oracle_lib):
+    """Thresholds are read four at a time and then one by one: 1 to 9 types, and thresholds that do not
+    ascend (a negative ratio)."""
+    sets = [[(1.0 / n, 8.0 + k, 2.0) for k in range(n)] for n in range(1, 10)]
+    sets.append([(0.5, 8.0, 2.0), (0.3, 9.0, 2.0), (0.3, 10.0, 2.0), (0.2, 11.0, 2.0), (-0.3, 12.0, 2.0)])
+    bins = [(700.0, 301), (60.0, 77)]
+    b = engine.batch([(bins, t, 40.0, 1.0, 60 + i) for i, t in enumerate(sets)])
+    b.run()
+    for i, t in enumerate(sets):
+        o = oracle_lib.simulate(bins, t, 40.0, 1.0, seed=60 + i, nthreads=0)
+        assert np.array_equal(b.result(i).per_type, o.per_type), i
+        assert np.array_equal(engine.simulate(bins, t, 40.0, 1.0, 60 + i).per_type, o.per_type), i
+    b.close()
