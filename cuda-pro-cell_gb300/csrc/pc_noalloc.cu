@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -261,8 +262,11 @@ extern "C" int pc_simulate_noalloc(const pc_bin* bins, uint64_t n_bins, const pc
   const uint32_t levels = std::min<uint32_t>(gmax, 40u) + 2u;
   const uint64_t per_buf_extra = align256(8ull * segs) + align256(8ull * (segs + 1)) + 256;
   uint64_t cells = 0;
-  if (fixed + 4096 < (uint64_t)PC_NOALLOC_SCRATCH_BYTES) {
-    const uint64_t room = (uint64_t)PC_NOALLOC_SCRATCH_BYTES - fixed - 4096;  // alignment slack
+  // alignment slack, less what the tree walk's fields add to the types (2 KB of it is enough): they
+  // take no input's room
+  const uint64_t slack = 4096 - (align256(sizeof(TypeDev) * n_types) - align256(offsetof(TypeDev, w_mean) * n_types));
+  if (fixed + slack < (uint64_t)PC_NOALLOC_SCRATCH_BYTES) {
+    const uint64_t room = (uint64_t)PC_NOALLOC_SCRATCH_BYTES - fixed - slack;
     if (room > levels * (per_buf_extra + 256)) cells = (room - levels * (per_buf_extra + 256)) / (8 + 16ull * levels);
   }
   if (cells < 4ull * segs + 1024) {

@@ -123,3 +123,26 @@ def test_noalloc_reports_sizes(built):
     many = [(2.5, 1)] * 2_000_000
     rc, _, _, _, err = noalloc_counts(many, [(1.0, 5.0, 1.0)], 10.0, 1.0, 1, 4_000_000)
     assert rc == 3 and "allocation-free scratch" in err
+
+
+def test_the_largest_input_the_array_takes(built):
+    """The limit on the input's size follows the rows, tables and counts that the sweeps need: per bin
+    16 + 4 + 8 B and its counts, per type 48 B, the sampler's tables, and level buffers of four cells
+    per segment. 64 types, one-cell bins that divide at most once."""
+    import torch
+    n_types, gens = 64, 2
+    segs = torch.cuda.get_device_properties(0).multi_processor_count * 8
+    r = lambda n: (n + 255) // 256 * 256  # noqa: E731
+
+    def fits(nb):
+        fixed = r(16 * nb) + r(4 * nb) + r(8 * (nb + 1)) + r(48 * n_types) + r(4 * 3073) + 256 + r(8 * gens * nb * n_types)
+        levels = 1 + 2
+        room = (64 << 20) - fixed - 4096 - levels * (r(8 * segs) + r(8 * (segs + 1)) + 512)
+        return room > 0 and room // (8 + 16 * levels) >= 4 * segs + 1024
+
+    most = max(nb for nb in range(50_000, 70_000) if fits(nb))
+    types = [(1.0 / n_types, 5.0 + 0.1 * k, 1.0) for k in range(n_types)]
+    for nb, want in ((most, 0), (most + 1, 3)):
+        rc, _, dims, _, err = noalloc_counts([(2.5, 1)] * nb, types, 10.0, 1.0, 1, gens * nb * n_types)
+        assert rc == want, (nb, err)
+        assert dims == (gens, nb, n_types)
