@@ -58,16 +58,19 @@ constexpr int kSigmaShift = 896;
 constexpr uint32_t kNarrowMaxGen = 31;
 constexpr double kMaxSigma = 0x1p127;
 
-// One cell type, in the descending-ratio order the reference samples in.
+// One cell type, in the descending-ratio order the reference samples in: what the level sweeps
+// read, and keep in shared memory.
 // The division sweep reads bytes 0-31 (mu, sigma, zlo, zhi, t_max) as two 16-byte loads.
-struct alignas(16) TypeDev {
+struct alignas(16) SweepType {
   double mu, sigma;  // 0, 8: mean, sd x 2^kSigmaShift (tau = fma(sd, z, mean))
   float zlo, zhi;    // 16: the FP32 z range for which fma(sigma, z, mu) > 0 (the truncation)
   double t_max;      // 24: its instance's t_max (read by the batched sweeps; plain: RunArgs)
   double cum;        // 32: cumulative ratio in this order
   int32_t mode;      // 40
   int32_t pad;
-  // the tree walk's form of the type (pc_walk.cuh; host_walk_type fills it)
+};
+// ... with the tree walk's form of the type (pc_walk.cuh; host_walk_type fills it).
+struct alignas(16) TypeDev : SweepType {
   float w_mean, w_sd;   // 48: mean, sd
   float w_eps;          // 56: an FP32 timer above it is certainly positive in FP64
   float w_band_gen;     // 60: error of the time left per generation of the phi cap
@@ -87,7 +90,7 @@ struct alignas(16) BatchType {
   uint32_t instance;    // 96
   uint32_t pad[3];
 };
-static_assert(sizeof(TypeDev) == 80 && sizeof(BatchType) == 112, "layout read by the division sweep");
+static_assert(sizeof(SweepType) == 48 && sizeof(TypeDev) == 80 && sizeof(BatchType) == 112, "layout read by the division sweep");
 
 struct InstanceDev {
   uint32_t type_begin, ntypes, fallback, pad;

@@ -19,7 +19,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -264,7 +263,7 @@ extern "C" int pc_simulate_noalloc(const pc_bin* bins, uint64_t n_bins, const pc
   uint64_t cells = 0;
   // alignment slack, less what the tree walk's fields add to the types (2 KB of it is enough): they
   // take no input's room
-  const uint64_t slack = 4096 - (align256(sizeof(TypeDev) * n_types) - align256(offsetof(TypeDev, w_mean) * n_types));
+  const uint64_t slack = 4096 - (align256(sizeof(TypeDev) * n_types) - align256(sizeof(SweepType) * n_types));
   if (fixed + slack < (uint64_t)PC_NOALLOC_SCRATCH_BYTES) {
     const uint64_t room = (uint64_t)PC_NOALLOC_SCRATCH_BYTES - fixed - slack;
     if (room > levels * (per_buf_extra + 256)) cells = (room - levels * (per_buf_extra + 256)) / (8 + 16ull * levels);

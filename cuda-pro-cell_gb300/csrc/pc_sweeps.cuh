@@ -89,7 +89,7 @@ __device__ __forceinline__ bool in_bounds(bool ok, uint32_t* error) {
 
 struct Smem {
   ZigTables zig;
-  TypeDev types[kMaxTypes];  // plain form only
+  SweepType types[kMaxTypes];  // plain form only
   __device__ __forceinline__ const ZigTables& zig_or(const RunArgs&) const { return zig; }
 };
 
@@ -100,8 +100,9 @@ __device__ __forceinline__ void stage(Smem& s, const RunArgs& a) {
   if (a.btypes) return;  // batched form: types come from the batch table
   const uint32_t* ts = reinterpret_cast<const uint32_t*>(a.types);
   uint32_t* td = reinterpret_cast<uint32_t*>(s.types);
-  const uint32_t nt = a.ntypes * (uint32_t)(sizeof(TypeDev) / 4);
-  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) td[i] = __ldg(ts + i);
+  constexpr uint32_t kWords = sizeof(SweepType) / 4, kStride = sizeof(TypeDev) / 4;
+  const uint32_t nt = a.ntypes * kWords;
+  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) td[i] = __ldg(ts + i / kWords * kStride + i % kWords);
 }
 
 // Rejection path of one daughter's normal: the generic ziggurat plus the truncation
@@ -176,7 +177,7 @@ struct TypeCtx {
 // The type's parameters from shared memory (plain form) or the batch table (batched form,
 // one entry per type of every instance), in three 16-byte loads at most.
 template <bool Batched>
-__device__ __forceinline__ TypeCtx type_ctx(const RunArgs& a, const TypeDev* smem_types, uint32_t ty) {
+__device__ __forceinline__ TypeCtx type_ctx(const RunArgs& a, const SweepType* smem_types, uint32_t ty) {
   TypeCtx c;
   if (Batched) {
     const uint4* q = reinterpret_cast<const uint4*>(a.btypes + ty);
@@ -190,7 +191,7 @@ __device__ __forceinline__ TypeCtx type_ctx(const RunArgs& a, const TypeDev* sme
     c.k1 = q5.y;
     c.root_begin = ((uint64_t)q5.w << 32) | q5.z;
   } else {
-    const TypeDev* t = smem_types + ty;
+    const SweepType* t = smem_types + ty;
     const double2 ms = *reinterpret_cast<const double2*>(&t->mu);
     const float2 z = *reinterpret_cast<const float2*>(&t->zlo);
     c.mu = ms.x;
@@ -357,10 +358,10 @@ __device__ void root_body(const RunArgs& a, const uint64_t root_base, const uint
                               : philox_ks(u32x4{0u, 0u, root, kPurposeRoot}, a.ks);
       const double u_type = unit53_closed_open(R.x, R.y);
       const double u_age = unit53_open_closed(R.z, R.w);
-      const TypeDev* types = Batched ? &a.btypes[type_begin].t : s.types;
-      const size_t tstride = Batched ? sizeof(BatchType) : sizeof(TypeDev);
-      auto type_at = [&](uint32_t i) -> const TypeDev& {
-        return *reinterpret_cast<const TypeDev*>(reinterpret_cast<const char*>(types) + i * tstride);
+      const SweepType* types = Batched ? &a.btypes[type_begin].t : s.types;
+      const size_t tstride = Batched ? sizeof(BatchType) : sizeof(SweepType);
+      auto type_at = [&](uint32_t i) -> const SweepType& {
+        return *reinterpret_cast<const SweepType*>(reinterpret_cast<const char*>(types) + i * tstride);
       };
       uint32_t ty = fallback;
       for (uint32_t i = 0; i < ntypes; ++i) {
@@ -375,7 +376,7 @@ __device__ void root_body(const RunArgs& a, const uint64_t root_base, const uint
         a.root_rec[rl] = (unsigned long long)cls | ((unsigned long long)(type_begin + ty) << 32) |
                          ((unsigned long long)(info & 0xFFu) << 48) |
                          ((unsigned long long)((info >> 8) & 3u) << 56);
-      const TypeDev& T = type_at(ty);
+      const SweepType& T = type_at(ty);
       bool leaf;
       if (T.mode == kModeQuiescent) {
         leaf = true;  // timer -1: out of time at once (cell.cu:69-75)
