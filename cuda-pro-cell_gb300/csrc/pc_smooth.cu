@@ -782,6 +782,7 @@ __global__ void __launch_bounds__(kThreads, !Kept      ? kBlocksDrawn
   __shared__ double u_age[kThreads];
   __shared__ __align__(8) float u_one[kThreads], u_one_lo[kThreads];
   constexpr uint32_t kWarps = kThreads / 32;
+  __shared__ uint32_t finite_lanes[kWarps];  // adjoint's pairs: candidates whose gradient is finite
   const uint32_t b = A.bin_order[blockIdx.x], k = blockIdx.z;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t slot = blockIdx.y * 32u + lane;
@@ -813,8 +814,11 @@ __global__ void __launch_bounds__(kThreads, !Kept      ? kBlocksDrawn
       if constexpr (Pairs) finite = finite && isfinite((float)a);
     }
     // A gradient that is not finite (FP32) is left out where a weight is 0, which walk() looks
-    // for and a pair does not: the whole block walks alone.
-    if constexpr (Pairs) finite = __syncthreads_and(finite) != 0;
+    // for and a pair does not: its candidate's lineages are walked alone.
+    if constexpr (Pairs) {
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, finite);
+      if (lane == 0u) finite_lanes[warp] = m;  // (grid_shared's barriers follow)
+    }
   }
   const double* my_prm = params + (uint64_t)(live ? c : 0u) * KQ + 3u * k;
   const double mu = live ? my_prm[1] : 0.0, sd = live ? my_prm[2] : 0.0;
@@ -830,6 +834,8 @@ __global__ void __launch_bounds__(kThreads, !Kept      ? kBlocksDrawn
   RemGrid rg;
   const bool grid = opaque(grid_shared(rg, mu, sd, A.t_max, steps, A.h, reinterpret_cast<float*>(u_age)));
   const RemFp64 rd{mu, sd, A.t_max, 0.0};
+  if constexpr (Backward && Pairs)
+    for (uint32_t w = 0; w < kWarps; ++w) finite = finite && ((finite_lanes[w] >> lane) & 1u) != 0u;
   const bool pairs = Pairs && opaque(grid && walks && finite && !quiescent && !fixed_tau);
   const RemGrid2 rg2(rg, rg);
   const float stop = stop_level(steps);  // once per block: the walks' stopping threshold

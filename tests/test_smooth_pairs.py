@@ -171,3 +171,28 @@ def test_adjoint_of_plans_with_a_deep_bin(engine, predraw, extra):
         engine.set_option("smooth_predraw", 1)
     terms = np.einsum("cv,cvkq->ckq", np.abs(g), np.abs(J))
     assert np.all(np.abs(both - alone) <= (64 * 64 + 2) * 2.0 ** -24 * terms + 1e-10)
+
+
+def test_a_neighbour_whose_gradient_is_not_finite(engine):
+    """It changes no other candidate's adjoint, not in the last bit."""
+    import torch
+    from procell.smooth import Smooth
+    rng = np.random.default_rng(12)
+    bins = [(float(v), int(f)) for v, f in zip(np.exp(rng.uniform(0, 8, 23)), rng.integers(1, 40, 23))]
+    sm = Smooth(engine, bins, n_types=2, t_max=140.0, phi=1.0, h=0.5, paths=1, seed=3)
+    P = np.empty((40, 2, 3))
+    P[..., 0] = rng.dirichlet(np.ones(2), 40)
+    P[..., 1] = rng.uniform(15, 60, (40, 2))
+    P[..., 2] = 0.3 * P[..., 1]
+    P = torch.tensor(P, device="cuda")
+    g = torch.tensor(rng.normal(size=(40, sm.n_values)), device="cuda")
+    want = sm.backward(P, g).cpu().numpy()
+    for odd in (0, 17, 39):
+        h = g.clone()
+        h[odd, ::5] = float("inf")
+        got = sm.backward(P, h).cpu().numpy()
+        others = np.arange(40) != odd
+        assert np.array_equal(got[others], want[others]), odd
+        assert not np.all(np.isfinite(got[odd]))
+    sm.sync()
+    sm.close()
